@@ -366,6 +366,180 @@ GL_HD uint64_t gl_shl(uint64_t x) {
   }
 }
 
+// ------------------------------------------------------------- lazy values
+//
+// The codelets add and subtract in three 32-bit limbs, x0 + x1*2^32 +
+// x2*2^64 with x2 signed, and reduce only where a value leaves the codelet or
+// meets a general product: an addition is one carry chain of three
+// instructions, where the canonical one is eight (8 ALU/FMA instructions for
+// gl_add, 5 for gl_sub), and a product by 2^k is a word shift and one or two
+// carry chains instead of a Montgomery product (9 ALU + 9 FMA).  The
+// generator (codegen.py) tracks the exact interval of every value, so x2
+// never overflows.  Measured on GB300 (issue cycles per warp and element in
+// a register loop, 64 registers): 16-point DFT 74.6 -> 40.0, 8-point 50.2 ->
+// 31.3, 15-point 109 -> 77, 17-point 167 -> 111; the ALU pipe is 93 % busy.
+struct gl_l3 {
+  uint32_t x0, x1, x2;
+};
+
+#if defined(__CUDACC__)
+// 2^32 - 1 from constant memory: as a literal the compiler turns the
+// multiply-adds below into shifts and subtractions (which measured 14 %
+// slower in the 16-point DFT: the ALU pipe is the busier one).
+static __device__ __constant__ uint32_t gl_c_eps = 0xffffffffu;
+#endif
+#ifndef GL_DEV_PTX
+inline gl_l3 gl_l_pack(unsigned __int128 v) {
+  return {(uint32_t)v, (uint32_t)(v >> 32), (uint32_t)(v >> 64)};
+}
+inline unsigned __int128 gl_l_value(const gl_l3 &a) {  // two's complement, sign-extended
+  return (unsigned __int128)(((__int128)(int32_t)a.x2 << 64)) + (((uint64_t)a.x1 << 32) | a.x0);
+}
+inline unsigned __int128 gl_l_value(uint64_t a) { return a; }
+#endif
+
+GL_HD gl_l3 gl_l3_of(const gl_l3 &a) { return a; }
+GL_HD gl_l3 gl_l3_of(uint64_t a) { return {(uint32_t)a, (uint32_t)(a >> 32), 0u}; }
+
+// a + b and a - b; either operand a 64-bit word (any value) or three limbs.
+template <class A, class B>
+GL_HD gl_l3 gl_ladd(const A &av, const B &bv) {
+#ifdef GL_DEV_PTX
+  const gl_l3 a = gl_l3_of(av), b = gl_l3_of(bv);
+  gl_l3 r;
+  asm("add.cc.u32 %0, %3, %6;\n\t"
+      "addc.cc.u32 %1, %4, %7;\n\t"
+      "addc.u32 %2, %5, %8;"
+      : "=&r"(r.x0), "=&r"(r.x1), "=r"(r.x2)
+      : "r"(a.x0), "r"(a.x1), "r"(a.x2), "r"(b.x0), "r"(b.x1), "r"(b.x2));
+  return r;
+#else
+  return gl_l_pack(gl_l_value(av) + gl_l_value(bv));
+#endif
+}
+template <class A, class B>
+GL_HD gl_l3 gl_lsub(const A &av, const B &bv) {
+#ifdef GL_DEV_PTX
+  const gl_l3 a = gl_l3_of(av), b = gl_l3_of(bv);
+  gl_l3 r;
+  asm("sub.cc.u32 %0, %3, %6;\n\t"
+      "subc.cc.u32 %1, %4, %7;\n\t"
+      "subc.u32 %2, %5, %8;"
+      : "=&r"(r.x0), "=&r"(r.x1), "=r"(r.x2)
+      : "r"(a.x0), "r"(a.x1), "r"(a.x2), "r"(b.x0), "r"(b.x1), "r"(b.x2));
+  return r;
+#else
+  return gl_l_pack(gl_l_value(av) - gl_l_value(bv));
+#endif
+}
+
+// a + M*p = a + M*2^64 - M*2^32 + M, 0 < M < 2^31: raises a value above zero.
+template <uint64_t M, class A>
+GL_HD gl_l3 gl_lbias(const A &av) {
+  static_assert(M > 0 && M < (1ull << 31), "bias out of range");
+  const gl_l3 k = {(uint32_t)M, 0u - (uint32_t)M, (uint32_t)M - 1};
+  return gl_ladd(av, k);
+}
+// M*p - a.
+template <uint64_t M, class A>
+GL_HD gl_l3 gl_lnegb(const A &av) {
+  static_assert(M < (1ull << 31), "bias out of range");
+  const gl_l3 k = {(uint32_t)M, 0u - (uint32_t)M, (uint32_t)M - (M > 0)};
+  return gl_lsub(k, av);
+}
+
+// A non-negative value (x2 < 2^31) to a 64-bit word congruent to it, not
+// necessarily below p: X + x2*(2^32 - 1), and a carry out of it is another
+// 2^32 - 1 (which cannot carry again: the wrapped sum is below 2^63).
+GL_HD uint64_t gl_lfold(const gl_l3 &a) {
+#ifdef GL_DEV_PTX
+  uint32_t r0, r1, c;
+  asm("mad.lo.cc.u32 %0, %5, %6, %3;\n\t"
+      "madc.hi.cc.u32 %1, %5, %6, %4;\n\t"
+      "addc.u32 %2, 0, 0;\n\t"
+      "sub.u32 %2, 0, %2;\n\t"
+      "add.cc.u32 %0, %0, %2;\n\t"
+      "addc.u32 %1, %1, 0;"
+      : "=&r"(r0), "=&r"(r1), "=&r"(c)
+      : "r"(a.x0), "r"(a.x1), "r"(a.x2), "r"(gl_c_eps));
+  return gl_pack(r0, r1);
+#else
+  const uint64_t x = ((uint64_t)a.x1 << 32) | a.x0, u = (uint64_t)a.x2 * GL_EPS, r = x + u;
+  return r < u ? r + GL_EPS : r;
+#endif
+}
+
+// The same for a signed x2, in three limbs (the new x2 is -1, 0 or 1): makes
+// room for a following shift.
+GL_HD gl_l3 gl_lnorm(const gl_l3 &a) {
+#ifdef GL_DEV_PTX
+  const uint32_t sg = (uint32_t)((int32_t)a.x2 >> 31);
+  gl_l3 r;
+  asm("sub.cc.u32 %0, %3, %5;\n\t"
+      "subc.cc.u32 %1, %4, %6;\n\t"
+      "subc.u32 %2, 0, %6;\n\t"
+      "add.cc.u32 %1, %1, %5;\n\t"
+      "addc.u32 %2, %2, %6;"
+      : "=&r"(r.x0), "=&r"(r.x1), "=&r"(r.x2)
+      : "r"(a.x0), "r"(a.x1), "r"(a.x2), "r"(sg));
+  return r;
+#else
+  const __int128 u = (__int128)(int32_t)a.x2 * (__int128)GL_EPS;
+  return gl_l_pack((((uint64_t)a.x1 << 32) | a.x0) + (unsigned __int128)u);
+#endif
+}
+
+// a * 2^K for 0 < K < 96, where a shifted by K mod 32 bits fits three limbs
+// (y0, y1, y2), y2 signed.  With 2^64 = 2^32 - 1 and 2^96 = -1:
+//   K < 32   the shifted limbs as they are;
+//   K < 64   y0*2^32 + y1*(2^32 - 1) - y2;
+//   K < 96   y0*(2^32 - 1) - y1 - y2*2^32.
+template <int K, class A>
+GL_HD gl_l3 gl_lshl(const A &av) {
+  static_assert(K > 0 && K < 96, "shift out of range");
+  constexpr int s = K % 32, q = K / 32;
+#ifdef GL_DEV_PTX
+  const gl_l3 x = gl_l3_of(av);
+  uint32_t y0 = x.x0, y1 = x.x1, y2 = x.x2;
+  if constexpr (s != 0) {
+    y0 = x.x0 << s;
+    y1 = __funnelshift_l(x.x0, x.x1, s);
+    y2 = __funnelshift_l(x.x1, x.x2, s);
+  }
+  gl_l3 r;
+  if constexpr (q == 0) {
+    r = {y0, y1, y2};
+  } else if constexpr (q == 1) {
+    const uint32_t sg = (uint32_t)((int32_t)y2 >> 31);
+    asm("mul.lo.u32 %0, %3, %4;\n\t"          // y1*EPS + y0*2^32, carry to x2
+        "mad.hi.cc.u32 %1, %3, %4, %5;\n\t"
+        "addc.u32 %2, 0, 0;\n\t"
+        "sub.cc.u32 %0, %0, %6;\n\t"
+        "subc.cc.u32 %1, %1, %7;\n\t"
+        "subc.u32 %2, %2, %7;"
+        : "=&r"(r.x0), "=&r"(r.x1), "=&r"(r.x2)
+        : "r"(y1), "r"(gl_c_eps), "r"(y0), "r"(y2), "r"(sg));
+  } else {
+    const uint32_t sg = (uint32_t)((int32_t)y2 >> 31);
+    asm("sub.cc.u32 %0, 0, %3;\n\t"           // y0*EPS >= 0
+        "subc.u32 %1, %3, 0;\n\t"
+        "sub.cc.u32 %0, %0, %4;\n\t"
+        "subc.cc.u32 %1, %1, %5;\n\t"
+        "subc.u32 %2, 0, %6;"
+        : "=&r"(r.x0), "=&r"(r.x1), "=&r"(r.x2)
+        : "r"(y0), "r"(y1), "r"(y2), "r"(sg));
+  }
+  return r;
+#else
+  const unsigned __int128 y = gl_l_value(av) << s;
+  const unsigned __int128 y0 = (uint32_t)y, y1 = (uint32_t)(y >> 32);
+  const unsigned __int128 y2 = (unsigned __int128)(__int128)(int32_t)(uint32_t)(y >> 64);
+  if (q == 0) return gl_l_pack(y);
+  if (q == 1) return gl_l_pack((y0 << 32) + y1 * GL_EPS - y2);
+  return gl_l_pack(y0 * GL_EPS - y1 - (y2 << 32));
+#endif
+}
+
 // x * 2^k mod p for a run-time k (any value; 2^192 = 1).
 GL_HD uint64_t gl_shl_rt(uint64_t x, uint32_t k) {
   k %= 192;

@@ -64,10 +64,6 @@ __device__ __forceinline__ void gl_gen_round1(const gl_pass_args &a, const gl_ge
       const uint64_t *p = src + (int64_t)(q.S1 * t) * a.in_is;
       x[t] = (live && j < a.in_limit) ? gl_ld_in(a, p, (a.flags & GL_PF_LOAD_CG) != 0) : 0;
     }
-    if ((a.flags & (GL_PF_CANON_IN | GL_PF_IN_TWIDDLE)) == GL_PF_CANON_IN) {
-#pragma unroll
-      for (int t = 0; t < R; t++) x[t] = gl_canon(x[t]);
-    }
     if ((a.flags & GL_PF_IN_TWIDDLE) && live) {
       const uint64_t col = (uint64_t)lane / a.tw_lane_div;
 #pragma unroll
@@ -76,7 +72,7 @@ __device__ __forceinline__ void gl_gen_round1(const gl_pass_args &a, const gl_ge
         if (j < a.in_limit) x[t] = gl_mont_mul(x[t], gl_tw2m(a.itw_lo, a.itw_hi, j * a.itw_jmul + col));
       }
     }
-    gl_dft<R, INV>(x);
+    gl_dft_lazy<R, INV>(x);
     if (q.NR == 1) {
       if (live) {
         uint64_t *dst = q.out + lane * a.out_ls;
@@ -86,7 +82,7 @@ __device__ __forceinline__ void gl_gen_round1(const gl_pass_args &a, const gl_ge
           uint64_t v = scale_all ? gl_mont_mul(x[t], a.tw_m[0]) : x[t];
           if (a.flags & GL_PF_PASS_TWIDDLE) v = gl_mont_mul(v, gl_pass_tw(a, col, t));
           if (a.flags & GL_PF_OUT_MUL) v = gl_out_mul(a, q.mul, lane, t, v);
-          gl_st_out(a, dst + (int64_t)t * a.out_is, v);
+          gl_st_out(a, dst + (int64_t)t * a.out_is, gl_canon(v));
         }
       }
     } else {
@@ -113,7 +109,7 @@ __device__ __forceinline__ void gl_gen_round2(const gl_pass_args &a, const gl_ge
     uint64_t x[R];
 #pragma unroll
     for (int t = 0; t < R; t++) x[t] = gl_sm_ld(a, sm, base + q.R3 * t, GL_GEN_LANES * q.LS);
-    gl_dft<R, INV>(x);
+    gl_dft_lazy<R, INV>(x);
 #pragma unroll
     for (int t = 0; t < R; t++) {
       uint64_t v = x[t];
@@ -145,7 +141,7 @@ __device__ __forceinline__ void gl_gen_round_last(const gl_pass_args &a, const g
     uint64_t x[R];
 #pragma unroll
     for (int t = 0; t < R; t++) x[t] = gl_sm_ld(a, sm, c * q.LS + base + t, GL_GEN_LANES * q.LS);
-    gl_dft<R, INV>(x);
+    gl_dft_lazy<R, INV>(x);
     const int64_t lane = q.lane0 + c;
     if (lane < (int64_t)a.lanes) {
       uint64_t *dst = q.out + lane * a.out_ls;
@@ -156,7 +152,7 @@ __device__ __forceinline__ void gl_gen_round_last(const gl_pass_args &a, const g
         uint64_t v = x[t];
         if (a.flags & GL_PF_PASS_TWIDDLE) v = gl_mont_mul(v, gl_pass_tw(a, col, k));
         if (a.flags & GL_PF_OUT_MUL) v = gl_out_mul(a, q.mul, lane, (int64_t)k, v);
-        gl_st_out(a, dst + (int64_t)k * a.out_is, v);
+        gl_st_out(a, dst + (int64_t)k * a.out_is, gl_canon(v));
       }
     }
   }

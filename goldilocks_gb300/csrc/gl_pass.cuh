@@ -27,7 +27,6 @@ enum : uint32_t {
   GL_PF_PTR_TABLE = 128u,      // batch item by = in_ptrs[by] / out_ptrs[by] (no *_bs)
   GL_PF_OUT_MUL = 256u,        // final store: outputs *= mul[...] (pointwise spectrum product)
   GL_PF_OUT_MUL_MONT = 512u,   // ... and * 2^-64 (product of two Montgomery words)
-  GL_PF_CANON_IN = 1024u,      // inputs may be >= p: reduce them on load (first pass of a call)
 };
 
 // Programmatic dependent launch (griddepcontrol, sm_90 and later).  A pass

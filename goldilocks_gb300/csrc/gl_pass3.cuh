@@ -20,7 +20,9 @@
 //
 // Each thread holds one radix-R group in registers (R <= 17), so the code per
 // round is one straight-line codelet and the kernel runs 1024 threads per
-// CTA.  Round 1 reads global memory directly and the last round writes it;
+// CTA.  The codelets take and give any words congruent to the values
+// (gl_dft_lazy): a twiddle product reduces them, and what leaves without one
+// is reduced on the store.  Round 1 reads global memory directly and the last round writes it;
 // rounds exchange through shared memory (XOR-swizzled against bank
 // conflicts).  Strides give the COL / ROW / FULL roles of gl_pass.cuh; the
 // same flags apply (pass twiddle, zero padding, coset factor, scale).
@@ -156,12 +158,6 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
           x[t] = (live && j < a.in_limit) ? gl_ld_in(a, src + (int64_t)(S1 * t) * a.in_is, false) : 0;
         }
       }
-      // Caller data may hold words >= p: the codelets' additions need canonical
-      // operands (the coset factor's Montgomery product reduces them anyway).
-      if ((a.flags & (GL_PF_CANON_IN | GL_PF_IN_TWIDDLE)) == GL_PF_CANON_IN) {
-#pragma unroll
-        for (int t = 0; t < R1; t++) x[t] = gl_canon(x[t]);
-      }
       if (a.flags & GL_PF_IN_TWIDDLE) {
         const uint64_t col = (uint64_t)lane / a.tw_lane_div;
 #pragma unroll
@@ -170,7 +166,7 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
           if (j < a.in_limit) x[t] = gl_mont_mul(x[t], gl_tw2m(a.itw_lo, a.itw_hi, j * a.itw_jmul + col));
         }
       }
-      gl_dft<R1, INV>(x);
+      gl_dft_lazy<R1, INV>(x);
       if constexpr (L::NR == 1) {
         // Single round: t is the output index.
         if (scale_all) {
@@ -191,7 +187,7 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
             for (int t = 0; t < R1; t++) gl_st_out(a, dst + (int64_t)t * a.out_is, gl_out_mul(a, mb, lane, t, x[t]));
           } else {
 #pragma unroll
-            for (int t = 0; t < R1; t++) gl_st_out(a, dst + (int64_t)t * a.out_is, x[t]);
+            for (int t = 0; t < R1; t++) gl_st_out(a, dst + (int64_t)t * a.out_is, gl_canon(x[t]));
           }
         }
       } else {
@@ -226,14 +222,14 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
         }
 #pragma unroll
         for (int t = 0; t < R2; t++) x[t] = gl_sm_ld(a, sm, L::word(c, pos[t]), LANES * L::LS);
-        gl_dft<R2, INV>(x);
+        gl_dft_lazy<R2, INV>(x);
 #pragma unroll
         for (int t = 0; t < R2; t++) gl_sm_st(a, sm, L::word(c, pos[t]), LANES * L::LS, x[t]);
         continue;
       }
 #pragma unroll
       for (int t = 0; t < R2; t++) x[t] = gl_sm_ld(a, sm, L::word(c, base + R3 * t), LANES * L::LS);
-      gl_dft<R2, INV>(x);
+      gl_dft_lazy<R2, INV>(x);
 #pragma unroll
       for (int t = 0; t < R2; t++) {
         uint64_t v = x[t];
@@ -278,7 +274,7 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
 #pragma unroll
         for (int t = 0; t < RL; t++) x[t] = gl_sm_ld(a, sm, L::word(c, base + t), LANES * L::LS);
       }
-      gl_dft<RL, INV>(x);
+      gl_dft_lazy<RL, INV>(x);
       const int64_t lane = lane0 + c;
       if constexpr (GT) {
         // Rows and column batches only: no pass twiddle in this form.
@@ -292,7 +288,7 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
           for (int t = 0; t < RL; t++) {
             int kk = kbase + (t * GTC::E3) % S1;
             if (kk >= S1) kk -= S1;
-            const uint64_t v = mul ? gl_out_mul(a, mb, lane, k1 + R1 * kk, x[t]) : x[t];
+            const uint64_t v = mul ? gl_out_mul(a, mb, lane, k1 + R1 * kk, x[t]) : gl_canon(x[t]);
             gl_st_out(a, dst + (int64_t)kk * kstride, v);
           }
         }
@@ -323,7 +319,7 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
             gl_st_out(a, dst + (int64_t)(kbase + SL * t) * a.out_is, gl_out_mul(a, mb, lane, kbase + SL * t, x[t]));
         } else {
 #pragma unroll
-          for (int t = 0; t < RL; t++) gl_st_out(a, dst + (int64_t)(kbase + SL * t) * a.out_is, x[t]);
+          for (int t = 0; t < RL; t++) gl_st_out(a, dst + (int64_t)(kbase + SL * t) * a.out_is, gl_canon(x[t]));
         }
       }
     }
