@@ -19,45 +19,58 @@
 // in round 3, so the gathers stay on distinct banks.)
 //
 // Each thread holds one radix-R group in registers (R <= 17), so the code per
-// round is one straight-line codelet and the kernel runs 1024 threads per
-// CTA.  The codelets take and give any words congruent to the values
-// (gl_dft_lazy): a twiddle product reduces them, and what leaves without one
-// is reduced on the store.  Round 1 reads global memory directly and the last round writes it;
-// rounds exchange through shared memory (XOR-swizzled against bank
-// conflicts).  Strides give the COL / ROW / FULL roles of gl_pass.cuh; the
-// same flags apply (pass twiddle, zero padding, coset factor, scale).
+// round is one straight-line codelet.  Round 1 reads global memory directly
+// and the last round writes it; rounds exchange through shared memory
+// (XOR-swizzled against bank conflicts).  Strides give the COL / ROW / FULL
+// roles of gl_pass.cuh; the same flags apply (pass twiddle, zero padding,
+// coset factor, scale).  The codelets take and give any words congruent to
+// the values (gl_dft_lazy); a twiddle product reduces them, and what leaves
+// without one is reduced on the store.
 #pragma once
 #include "gl_pass.cuh"
 
 template <int R1, int R2, int R3, int LANES>
 struct gl_p3_layout {
   static constexpr int M = R1 * R2 * R3;
+  static constexpr int S1 = R2 * R3;
   static constexpr int NR = R2 == 1 ? 1 : (R3 == 1 ? 2 : 3);
   static constexpr int RL = NR == 3 ? R3 : (NR == 2 ? R2 : R1);  // last radix
   static constexpr bool POW2 = (RL & (RL - 1)) == 0 && (M & (M - 1)) == 0;
   static constexpr int SH = RL == 16 ? 4 : RL == 8 ? 3 : RL == 4 ? 2 : RL == 2 ? 1 : 0;
   static constexpr int MSK = POW2 ? (RL < 16 ? RL - 1 : 15) : 0;
-  // Lane stride: a multiple of 16 words plus 16 / min(LANES, 16).  A
-  // half-warp's 16 accesses (64-bit words; 16 words per 128-byte wavefront)
+  // A half-warp's 16 accesses (64-bit words; 16 words per 128-byte wavefront)
   // cover 16 / LANES positions of each of LANES lanes, so the lanes must fall
-  // on distinct word residues mod 16: +4 for four lanes, +8 for two, +2 for
-  // eight, an odd stride for 16 or more (a model of the access pattern of the
-  // three rounds puts each of these at one wavefront per half-warp where the
-  // old +4 for every lane count took two to four).
-  static constexpr int LS = ((M + 15) / 16) * 16 + 16 / (LANES < 16 ? LANES : 16);
+  // on distinct word residues mod 16, LSTEP apart: by an XOR of the word
+  // index in the power-of-two tiles, by the lane stride in the others (odd
+  // for 16 lanes or more).
+  static constexpr int LSTEP = 16 / (LANES < 16 ? LANES : 16);
+  static constexpr int LS = POW2 ? M : ((M + 15) / 16) * 16 + LSTEP;
+  static_assert(!POW2 || NR == 1 || M % 16 == 0, "power-of-two tiles are whole 16-word blocks");
+  // Word of position p of lane c.
   static __device__ __forceinline__ int word(int c, int p) {
-    return c * LS + (POW2 ? (p ^ ((p >> SH) & MSK)) : p);
+    return POW2 ? c * LS + (p ^ ((p >> SH) & MSK) ^ ((c * LSTEP) & 15)) : c * LS + p;
+  }
+  // Word of position pb + tb from base = word(c, pb), where tb is a multiple
+  // of the digit a round walks and shares no bit with pb: the swizzle is
+  // linear over XOR, so the step is an XOR of the low four bits with a
+  // constant and an immediate offset.  (Evaluating word() for every access
+  // took three to four instructions each, 16 of the 259 per element of the
+  // 4096-point column pass.)
+  static __device__ __forceinline__ int at(int base, int tb) {
+    const int w = tb ^ ((tb >> SH) & MSK);
+    return POW2 ? (base ^ (w & 15)) + (w & ~15) : base + tb;
   }
   // Shared memory after the tile (words), staged before round 1 and
-  // published by the barrier that ends it:
-  //   T2    the round-2 twiddles tw_r2[R1*i], i < R2*R3 (three rounds, the
-  //         Cooley-Tukey form only);
+  // published by the barrier that ends it.  Three rounds (the Cooley-Tukey
+  // form):
+  //   T2    the round-2 twiddles omega_(R2 R3)^(d3*k2) at [k2*R3 + d3];
+  // two or three rounds:
   //   STEP  per lane c and last-round output digit t, the pass-twiddle step
   //         omega_n^(col_c * SL * t) (SL: output stride of the last digit),
   //         RL + 1 words per lane so that the lanes fall on distinct banks.
   static constexpr int TILE = NR == 1 ? 0 : LANES * LS;
   static constexpr int T2 = TILE;
-  static constexpr int NT2 = NR == 3 ? R2 * R3 : 0;
+  static constexpr int NT2 = NR == 3 ? S1 : 0;
   static constexpr int STEP = T2 + NT2;
   static constexpr int SS = RL + 1;  // per-lane stride: lanes on distinct banks
   static constexpr int NSTEP = NR == 1 ? 0 : LANES * SS;
@@ -85,6 +98,13 @@ struct gl_gt_consts {
   static constexpr int E3 = R2 * BINV;                 // 0 mod R2, 1 mod R3
 };
 
+// A round's groups over the CTA's threads: idx = threadIdx.x + it*NT, without
+// a bound check where the groups fill every pass over them.
+#define GL_ROUND(idx, COUNT)                                                                       \
+  _Pragma("unroll 1") for (int gl_it = 0, idx = threadIdx.x; gl_it < ((COUNT) + NT - 1) / NT;      \
+                           gl_it++, idx += NT)                                                     \
+    if ((COUNT) % NT == 0 || idx < (COUNT))
+
 // One CTA's work: tile (bx, by, bz) of the pass described by `a`, with NT
 // threads and the dynamic shared memory `sm`.  Called by gl_pass3_kernel
 // (tile = blockIdx) and by the persistent batch kernel (tile from its queue).
@@ -95,26 +115,28 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   using GTC = gl_gt_consts<R2, R3>;
   constexpr int M = L::M;
   constexpr int S1 = R2 * R3;
+  constexpr int TILE = LANES * L::LS;
   static_assert(!GT || (L::NR == 3 && gl_gcd(R2, R3) == 1), "Good-Thomas inner transform needs coprime R2, R3");
 
   const int64_t lane0 = bx * LANES;
   gl_pdl_launch_dependents();
 
-  // Stage the round-2 twiddles and the pass-twiddle steps (read after the
-  // barrier that ends round 1).  They come from constant tables, so they are
-  // loaded before the wait below and their latency overlaps the previous
-  // pass's tail (under programmatic dependent launch) and this pass's loads.
+  // Stage the tables (read after the barrier that ends round 1).  They come
+  // from constant tables, so they are loaded before the wait below and their
+  // latency overlaps the previous pass's tail (under programmatic dependent
+  // launch) and this pass's loads.
   constexpr int SL = L::NR == 3 ? R1 * R2 : R1;  // output stride of the last digit
   const bool tw_steps = (a.flags & (GL_PF_PASS_TWIDDLE | GL_PF_TW_TABLE)) == GL_PF_PASS_TWIDDLE;
+  if constexpr (L::NR == 3 && !GT) {
+    for (int i = threadIdx.x; i < S1; i += NT)
+      gl_sm_st(a, sm, L::T2 + i, L::WORDS, __ldg(a.tw_r2 + R1 * (i % R3) * (i / R3)));
+  }
   if constexpr (L::NR > 1) {
-    if constexpr (L::NT2 > 0 && !GT) {
-      for (int i = threadIdx.x; i < L::NT2; i += NT) gl_sm_st(a, sm, L::T2 + i, L::WORDS, __ldg(a.tw_r2 + R1 * i));
-    }
     if (tw_steps) {
       for (int i = threadIdx.x; i < L::NSTEP; i += NT) {
         const int c = i / L::SS, t = i % L::SS;
         if (t >= L::RL) continue;
-        if (lane0 + c >= (int64_t)a.lanes) continue;  // lanes past the end read no table
+        if (lane0 + c >= (int64_t)a.lanes) continue;
         const uint64_t col = (uint64_t)(lane0 + c) / a.tw_lane_div + a.tw_col0;
         uint64_t v = gl_tw2m(a.tw_lo, a.tw_hi, col * (uint64_t)(SL * t));
         if (a.tw_unscale) v = gl_mont_mul(v, a.tw_unscale);
@@ -132,11 +154,14 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   const bool scale_all = (a.flags & GL_PF_SCALE_ALL) != 0;
   const bool load_lane_fast = (a.flags & GL_PF_LOAD_LANE_FAST) != 0;
   const bool store_lane_fast = (a.flags & GL_PF_STORE_LANE_FAST) != 0;
+  const bool load_cg = (a.flags & GL_PF_LOAD_CG) != 0;  // written earlier in the same launch: read via L2
+  // Every lane and index of the tile is there (uniform over the CTA).
+  const bool whole = lane0 + LANES <= (int64_t)a.lanes && a.in_limit >= (uint32_t)M;
 
   // ------------------------------------------------------------- round 1
   {
     constexpr int G = M / R1;  // groups per lane: jB = (d2, d3)
-    for (int idx = threadIdx.x; idx < LANES * G; idx += NT) {
+    GL_ROUND(idx, LANES * G) {
       int c, g;
       if (load_lane_fast) { c = idx % LANES; g = idx / LANES; }
       else { g = idx % G; c = idx / G; }
@@ -144,18 +169,15 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
       const bool live = lane < (int64_t)a.lanes;
       uint64_t x[R1];
       const uint64_t *src = in + lane * a.in_ls + (int64_t)g * a.in_is;
-      if (a.flags & GL_PF_LOAD_CG) {
-        // Input written earlier in the same launch by other CTAs: read via L2.
+      const int64_t step = (int64_t)S1 * a.in_is;
+      if (whole && !load_cg) {
 #pragma unroll
-        for (int t = 0; t < R1; t++) {
-          const uint32_t j = (uint32_t)(g + S1 * t);
-          x[t] = (live && j < a.in_limit) ? gl_ld_in(a, src + (int64_t)(S1 * t) * a.in_is, true) : 0;
-        }
+        for (int t = 0; t < R1; t++) x[t] = gl_ld_in(a, src + t * step, false);
       } else {
 #pragma unroll
         for (int t = 0; t < R1; t++) {
           const uint32_t j = (uint32_t)(g + S1 * t);
-          x[t] = (live && j < a.in_limit) ? gl_ld_in(a, src + (int64_t)(S1 * t) * a.in_is, false) : 0;
+          x[t] = (live && j < a.in_limit) ? gl_ld_in(a, src + t * step, load_cg) : 0;
         }
       }
       if (a.flags & GL_PF_IN_TWIDDLE) {
@@ -191,11 +213,12 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
           }
         }
       } else {
+        const int base = L::word(c, g);
 #pragma unroll
         for (int t = 0; t < R1; t++) {
           uint64_t v = x[t];
-          if (t > 0 || scale_all) v = gl_mont_mul(v, __ldg(a.tw_m + g * t));
-          gl_sm_st(a, sm, L::word(c, g + S1 * t), LANES * L::LS, v);
+          if (t > 0 || scale_all) v = gl_mont_mul(v, __ldg(a.tw_m + (uint32_t)(g * t)));
+          gl_sm_st(a, sm, L::at(base, S1 * t), TILE, v);
         }
       }
     }
@@ -206,10 +229,9 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   // ------------------------------------------------------------- round 2
   if constexpr (L::NR == 3) {
     constexpr int G = R1 * R3;  // groups (k1, d3)
-    for (int idx = threadIdx.x; idx < LANES * G; idx += NT) {
+    GL_ROUND(idx, LANES * G) {
       const int c = idx % LANES, g = idx / LANES;
       const int k1 = g / R3, d3 = g % R3;
-      const int base = k1 * S1 + d3;
       uint64_t x[R2];
       if constexpr (GT) {
         // inputs a at (R3*a + R2*b) mod S1, b = d3; outputs k2 = t in their place
@@ -218,23 +240,25 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
         for (int t = 0; t < R2; t++) {
           int v = R2 * d3 + R3 * t;
           if (v >= S1) v -= S1;
-          pos[t] = k1 * S1 + v;
+          pos[t] = L::word(c, k1 * S1 + v);
         }
 #pragma unroll
-        for (int t = 0; t < R2; t++) x[t] = gl_sm_ld(a, sm, L::word(c, pos[t]), LANES * L::LS);
+        for (int t = 0; t < R2; t++) x[t] = gl_sm_ld(a, sm, pos[t], TILE);
         gl_dft_lazy<R2, INV>(x);
 #pragma unroll
-        for (int t = 0; t < R2; t++) gl_sm_st(a, sm, L::word(c, pos[t]), LANES * L::LS, x[t]);
-        continue;
-      }
+        for (int t = 0; t < R2; t++) gl_sm_st(a, sm, pos[t], TILE, x[t]);
+      } else {
+        const int base = L::word(c, k1 * S1 + d3);
+        const int tw = L::T2 + d3;
 #pragma unroll
-      for (int t = 0; t < R2; t++) x[t] = gl_sm_ld(a, sm, L::word(c, base + R3 * t), LANES * L::LS);
-      gl_dft_lazy<R2, INV>(x);
+        for (int t = 0; t < R2; t++) x[t] = gl_sm_ld(a, sm, L::at(base, R3 * t), TILE);
+        gl_dft_lazy<R2, INV>(x);
 #pragma unroll
-      for (int t = 0; t < R2; t++) {
-        uint64_t v = x[t];
-        if (t > 0) v = gl_mont_mul(v, gl_sm_ld(a, sm, L::T2 + d3 * t, L::WORDS));
-        gl_sm_st(a, sm, L::word(c, base + R3 * t), LANES * L::LS, v);
+        for (int t = 0; t < R2; t++) {
+          uint64_t v = x[t];
+          if (t > 0) v = gl_mont_mul(v, gl_sm_ld(a, sm, tw + R3 * t, L::WORDS));
+          gl_sm_st(a, sm, L::at(base, R3 * t), TILE, v);
+        }
       }
     }
     __syncthreads();
@@ -244,82 +268,73 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   {
     constexpr int RL = L::RL;
     constexpr int G = M / RL;                      // groups: (k1, k2) or k1
-    for (int idx = threadIdx.x; idx < LANES * G; idx += NT) {
+    GL_ROUND(idx, LANES * G) {
       int c, g;
       if (store_lane_fast) { c = idx % LANES; g = idx / LANES; }
       else { g = idx % G; c = idx / G; }
       // group g enumerates (k1, k2) with k2 fastest for 3 rounds (positions
       // k1*S1 + k2*R3 + t), or k1 for 2 rounds (positions k1*R2 + t).
-      int base, kbase;
-      if constexpr (L::NR == 3) {
-        const int k1 = g / R2, k2 = g % R2;
-        base = k1 * S1 + k2 * R3;
-        // GT: k = k1 + R1 * ((k2 * E2 + t * E3) mod S1); kbase holds k2 * E2 mod S1
-        kbase = GT ? (k2 * GTC::E2) % S1 : k1 + R1 * k2;
-      } else {
-        base = g * R2;
-        kbase = g;
-      }
+      const int k1 = L::NR == 3 ? g / R2 : g, k2 = L::NR == 3 ? g % R2 : 0;
       uint64_t x[RL];
       if constexpr (GT) {
         // inputs b at (R3*k2 + R2*b) mod S1 of block k1
-        const int k1 = g / R2, k2 = g % R2;
 #pragma unroll
         for (int t = 0; t < RL; t++) {
           int v = R3 * k2 + R2 * t;
           if (v >= S1) v -= S1;
-          x[t] = gl_sm_ld(a, sm, L::word(c, k1 * S1 + v), LANES * L::LS);
+          x[t] = gl_sm_ld(a, sm, L::word(c, k1 * S1 + v), TILE);
         }
       } else {
+        const int base = L::word(c, g * RL);
 #pragma unroll
-        for (int t = 0; t < RL; t++) x[t] = gl_sm_ld(a, sm, L::word(c, base + t), LANES * L::LS);
+        for (int t = 0; t < RL; t++) x[t] = gl_sm_ld(a, sm, L::at(base, t), TILE);
       }
       gl_dft_lazy<RL, INV>(x);
       const int64_t lane = lane0 + c;
+      if (lane >= (int64_t)a.lanes) continue;
+      uint64_t *dst = out + lane * a.out_ls;
       if constexpr (GT) {
         // Rows and column batches only: no pass twiddle in this form.
-        if (lane < (int64_t)a.lanes) {
-          const int k1 = g / R2;
-          uint64_t *dst = out + lane * a.out_ls + (int64_t)k1 * a.out_is;
-          const int64_t kstride = (int64_t)R1 * a.out_is;
-          const bool mul = (a.flags & GL_PF_OUT_MUL) != 0;
-          const uint64_t *mb = mul ? a.mul + by * a.mul_bs + bz * a.mul_bs2 : nullptr;
+        // k = k1 + R1 * ((k2 * E2 + t * E3) mod S1)
+        const int kbase = (k2 * GTC::E2) % S1;
+        dst += (int64_t)k1 * a.out_is;
+        const int64_t kstride = (int64_t)R1 * a.out_is;
+        const bool mul = (a.flags & GL_PF_OUT_MUL) != 0;
+        const uint64_t *mb = mul ? a.mul + by * a.mul_bs + bz * a.mul_bs2 : nullptr;
 #pragma unroll
-          for (int t = 0; t < RL; t++) {
-            int kk = kbase + (t * GTC::E3) % S1;
-            if (kk >= S1) kk -= S1;
-            const uint64_t v = mul ? gl_out_mul(a, mb, lane, k1 + R1 * kk, x[t]) : gl_canon(x[t]);
-            gl_st_out(a, dst + (int64_t)kk * kstride, v);
-          }
+        for (int t = 0; t < RL; t++) {
+          int kk = kbase + (t * GTC::E3) % S1;
+          if (kk >= S1) kk -= S1;
+          const uint64_t v = mul ? gl_out_mul(a, mb, lane, k1 + R1 * kk, x[t]) : gl_canon(x[t]);
+          gl_st_out(a, dst + (int64_t)kk * kstride, v);
         }
-        continue;
-      }
-      if (lane < (int64_t)a.lanes) {
-        uint64_t *dst = out + lane * a.out_ls;
+      } else {
+        const int kbase = k1 + R1 * k2;  // output index of t: kbase + SL*t
+        dst += (int64_t)kbase * a.out_is;
+        const int64_t kstep = (int64_t)SL * a.out_is;
         if (tw_steps) {
           // tw(col, kbase + SL*t) = tw(col, kbase) * omega_n^(col*SL*t).
           const uint64_t col = (uint64_t)lane / a.tw_lane_div + a.tw_col0;
-          const uint64_t base = gl_tw2m(a.tw_lo, a.tw_hi, col * (uint64_t)kbase);
+          const uint64_t first = gl_tw2m(a.tw_lo, a.tw_hi, col * (uint64_t)kbase);
 #pragma unroll
           for (int t = 0; t < RL; t++) {
-            const uint64_t tw = t == 0 ? base : gl_mont_mul(base, gl_sm_ld(a, sm, L::STEP + c * L::SS + t, L::WORDS));
-            gl_st_out(a, dst + (int64_t)(kbase + SL * t) * a.out_is, gl_mont_mul(x[t], tw));
+            const uint64_t tw =
+                t == 0 ? first : gl_mont_mul(first, gl_sm_ld(a, sm, L::STEP + c * L::SS + t, L::WORDS));
+            gl_st_out(a, dst + t * kstep, gl_mont_mul(x[t], tw));
           }
         } else if (a.flags & GL_PF_PASS_TWIDDLE) {
           const uint64_t col = (uint64_t)lane / a.tw_lane_div;
 #pragma unroll
-          for (int t = 0; t < RL; t++) {
-            const uint64_t k = (uint64_t)(kbase + SL * t);
-            gl_st_out(a, dst + (int64_t)k * a.out_is, gl_mont_mul(x[t], gl_pass_tw(a, col, k)));
-          }
+          for (int t = 0; t < RL; t++)
+            gl_st_out(a, dst + t * kstep, gl_mont_mul(x[t], gl_pass_tw(a, col, (uint64_t)(kbase + SL * t))));
         } else if (a.flags & GL_PF_OUT_MUL) {
           const uint64_t *mb = a.mul + by * a.mul_bs + bz * a.mul_bs2;
 #pragma unroll
           for (int t = 0; t < RL; t++)
-            gl_st_out(a, dst + (int64_t)(kbase + SL * t) * a.out_is, gl_out_mul(a, mb, lane, kbase + SL * t, x[t]));
+            gl_st_out(a, dst + t * kstep, gl_out_mul(a, mb, lane, kbase + SL * t, x[t]));
         } else {
 #pragma unroll
-          for (int t = 0; t < RL; t++) gl_st_out(a, dst + (int64_t)(kbase + SL * t) * a.out_is, gl_canon(x[t]));
+          for (int t = 0; t < RL; t++) gl_st_out(a, dst + t * kstep, gl_canon(x[t]));
         }
       }
     }
