@@ -47,7 +47,7 @@ struct gl_p3_layout {
   static constexpr int LS = POW2 ? M : ((M + 15) / 16) * 16 + LSTEP;
   static_assert(!POW2 || NR == 1 || M % 16 == 0, "power-of-two tiles are whole 16-word blocks");
   // Word of position p of lane c.
-  static __device__ __forceinline__ int word(int c, int p) {
+  static __device__ __forceinline__ uint32_t word(uint32_t c, uint32_t p) {
     return POW2 ? c * LS + (p ^ ((p >> SH) & MSK) ^ ((c * LSTEP) & 15)) : c * LS + p;
   }
   // Word of position pb + tb from base = word(c, pb), where tb is a multiple
@@ -56,9 +56,9 @@ struct gl_p3_layout {
   // constant and an immediate offset.  (Evaluating word() for every access
   // took three to four instructions each, 16 of the 259 per element of the
   // 4096-point column pass.)
-  static __device__ __forceinline__ int at(int base, int tb) {
-    const int w = tb ^ ((tb >> SH) & MSK);
-    return POW2 ? (base ^ (w & 15)) + (w & ~15) : base + tb;
+  static __device__ __forceinline__ uint32_t at(uint32_t base, uint32_t tb) {
+    const uint32_t w = tb ^ ((tb >> SH) & MSK);
+    return POW2 ? (base ^ (w & 15u)) + (w & ~15u) : base + tb;
   }
   // Shared memory after the tile (words), staged before round 1 and
   // published by the barrier that ends it.  Three rounds (the Cooley-Tukey
@@ -101,7 +101,7 @@ struct gl_gt_consts {
 // A round's groups over the CTA's threads: idx = threadIdx.x + it*NT, without
 // a bound check where the groups fill every pass over them.
 #define GL_ROUND(idx, COUNT)                                                                       \
-  _Pragma("unroll 1") for (int gl_it = 0, idx = threadIdx.x; gl_it < ((COUNT) + NT - 1) / NT;      \
+  _Pragma("unroll 1") for (uint32_t gl_it = 0, idx = threadIdx.x; gl_it < ((COUNT) + NT - 1) / NT;      \
                            gl_it++, idx += NT)                                                     \
     if ((COUNT) % NT == 0 || idx < (COUNT))
 
@@ -118,7 +118,12 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   constexpr int TILE = LANES * L::LS;
   static_assert(!GT || (L::NR == 3 && gl_gcd(R2, R3) == 1), "Good-Thomas inner transform needs coprime R2, R3");
 
-  const int64_t lane0 = bx * LANES;
+  // Lanes, groups and positions are 32-bit (a pass has fewer than 2^32 lanes);
+  // only addresses are 64-bit.  The lane's column index is a division only
+  // for interleaved columns: as a 64-bit division in each thread it cost up
+  // to ten instructions per element.
+  const uint32_t lane0 = (uint32_t)bx * LANES;
+  auto column = [&](uint32_t lane) { return a.tw_lane_div == 1 ? lane : lane / a.tw_lane_div; };
   gl_pdl_launch_dependents();
 
   // Stage the tables (read after the barrier that ends round 1).  They come
@@ -133,12 +138,12 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   }
   if constexpr (L::NR > 1) {
     if (tw_steps) {
-      for (int i = threadIdx.x; i < L::NSTEP; i += NT) {
-        const int c = i / L::SS, t = i % L::SS;
+      for (uint32_t i = threadIdx.x; i < L::NSTEP; i += NT) {
+        const uint32_t c = i / L::SS, t = i % L::SS;
         if (t >= L::RL) continue;
-        if (lane0 + c >= (int64_t)a.lanes) continue;
-        const uint64_t col = (uint64_t)(lane0 + c) / a.tw_lane_div + a.tw_col0;
-        uint64_t v = gl_tw2m(a.tw_lo, a.tw_hi, col * (uint64_t)(SL * t));
+        if (lane0 + c >= a.lanes) continue;  // lanes past the end read no table
+        const uint64_t col = column(lane0 + c) + a.tw_col0;
+        uint64_t v = gl_tw2m(a.tw_lo, a.tw_hi, col * (uint32_t)(SL * t));
         if (a.tw_unscale) v = gl_mont_mul(v, a.tw_unscale);
         gl_sm_st(a, sm, L::STEP + i, L::WORDS, v);
       }
@@ -156,19 +161,19 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   const bool store_lane_fast = (a.flags & GL_PF_STORE_LANE_FAST) != 0;
   const bool load_cg = (a.flags & GL_PF_LOAD_CG) != 0;  // written earlier in the same launch: read via L2
   // Every lane and index of the tile is there (uniform over the CTA).
-  const bool whole = lane0 + LANES <= (int64_t)a.lanes && a.in_limit >= (uint32_t)M;
+  const bool whole = lane0 + LANES <= a.lanes && lane0 + LANES > lane0 && a.in_limit >= (uint32_t)M;
 
   // ------------------------------------------------------------- round 1
   {
-    constexpr int G = M / R1;  // groups per lane: jB = (d2, d3)
+    constexpr uint32_t G = M / R1;  // groups per lane: jB = (d2, d3)
     GL_ROUND(idx, LANES * G) {
-      int c, g;
+      uint32_t c, g;
       if (load_lane_fast) { c = idx % LANES; g = idx / LANES; }
       else { g = idx % G; c = idx / G; }
-      const int64_t lane = lane0 + c;
-      const bool live = lane < (int64_t)a.lanes;
+      const uint32_t lane = lane0 + c;
+      const bool live = lane < a.lanes;
       uint64_t x[R1];
-      const uint64_t *src = in + lane * a.in_ls + (int64_t)g * a.in_is;
+      const uint64_t *src = in + (uint64_t)a.in_ls * lane + (uint64_t)a.in_is * g;
       const int64_t step = (int64_t)S1 * a.in_is;
       if (whole && !load_cg) {
 #pragma unroll
@@ -176,15 +181,15 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
       } else {
 #pragma unroll
         for (int t = 0; t < R1; t++) {
-          const uint32_t j = (uint32_t)(g + S1 * t);
+          const uint32_t j = g + S1 * t;
           x[t] = (live && j < a.in_limit) ? gl_ld_in(a, src + t * step, load_cg) : 0;
         }
       }
       if (a.flags & GL_PF_IN_TWIDDLE) {
-        const uint64_t col = (uint64_t)lane / a.tw_lane_div;
+        const uint32_t col = column(lane);
 #pragma unroll
         for (int t = 0; t < R1; t++) {
-          const uint64_t j = (uint64_t)(g + S1 * t);
+          const uint32_t j = g + S1 * t;
           if (j < a.in_limit) x[t] = gl_mont_mul(x[t], gl_tw2m(a.itw_lo, a.itw_hi, j * a.itw_jmul + col));
         }
       }
@@ -197,9 +202,9 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
           for (int t = 0; t < R1; t++) x[t] = gl_mont_mul(x[t], s);
         }
         if (live) {
-          uint64_t *dst = out + lane * a.out_ls;
+          uint64_t *dst = out + (uint64_t)a.out_ls * lane;
           if (a.flags & GL_PF_PASS_TWIDDLE) {
-            const uint64_t col = (uint64_t)lane / a.tw_lane_div;
+            const uint64_t col = column(lane);
 #pragma unroll
             for (int t = 0; t < R1; t++)
               gl_st_out(a, dst + (int64_t)t * a.out_is, gl_mont_mul(x[t], gl_pass_tw(a, col, t)));
@@ -213,11 +218,11 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
           }
         }
       } else {
-        const int base = L::word(c, g);
+        const uint32_t base = L::word(c, g);
 #pragma unroll
         for (int t = 0; t < R1; t++) {
           uint64_t v = x[t];
-          if (t > 0 || scale_all) v = gl_mont_mul(v, __ldg(a.tw_m + (uint32_t)(g * t)));
+          if (t > 0 || scale_all) v = gl_mont_mul(v, __ldg(a.tw_m + g * t));
           gl_sm_st(a, sm, L::at(base, S1 * t), TILE, v);
         }
       }
@@ -228,10 +233,10 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
 
   // ------------------------------------------------------------- round 2
   if constexpr (L::NR == 3) {
-    constexpr int G = R1 * R3;  // groups (k1, d3)
+    constexpr uint32_t G = R1 * R3;  // groups (k1, d3)
     GL_ROUND(idx, LANES * G) {
-      const int c = idx % LANES, g = idx / LANES;
-      const int k1 = g / R3, d3 = g % R3;
+      const uint32_t c = idx % LANES, g = idx / LANES;
+      const uint32_t k1 = g / R3, d3 = g % R3;
       uint64_t x[R2];
       if constexpr (GT) {
         // inputs a at (R3*a + R2*b) mod S1, b = d3; outputs k2 = t in their place
@@ -248,8 +253,8 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
 #pragma unroll
         for (int t = 0; t < R2; t++) gl_sm_st(a, sm, pos[t], TILE, x[t]);
       } else {
-        const int base = L::word(c, k1 * S1 + d3);
-        const int tw = L::T2 + d3;
+        const uint32_t base = L::word(c, k1 * S1 + d3);
+        const uint32_t tw = L::T2 + d3;
 #pragma unroll
         for (int t = 0; t < R2; t++) x[t] = gl_sm_ld(a, sm, L::at(base, R3 * t), TILE);
         gl_dft_lazy<R2, INV>(x);
@@ -267,14 +272,14 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   // ------------------------------------------------------- last round
   {
     constexpr int RL = L::RL;
-    constexpr int G = M / RL;                      // groups: (k1, k2) or k1
+    constexpr uint32_t G = M / RL;                 // groups: (k1, k2) or k1
     GL_ROUND(idx, LANES * G) {
-      int c, g;
+      uint32_t c, g;
       if (store_lane_fast) { c = idx % LANES; g = idx / LANES; }
       else { g = idx % G; c = idx / G; }
       // group g enumerates (k1, k2) with k2 fastest for 3 rounds (positions
       // k1*S1 + k2*R3 + t), or k1 for 2 rounds (positions k1*R2 + t).
-      const int k1 = L::NR == 3 ? g / R2 : g, k2 = L::NR == 3 ? g % R2 : 0;
+      const uint32_t k1 = L::NR == 3 ? g / R2 : g, k2 = L::NR == 3 ? g % R2 : 0;
       uint64_t x[RL];
       if constexpr (GT) {
         // inputs b at (R3*k2 + R2*b) mod S1 of block k1
@@ -285,19 +290,19 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
           x[t] = gl_sm_ld(a, sm, L::word(c, k1 * S1 + v), TILE);
         }
       } else {
-        const int base = L::word(c, g * RL);
+        const uint32_t base = L::word(c, g * RL);
 #pragma unroll
         for (int t = 0; t < RL; t++) x[t] = gl_sm_ld(a, sm, L::at(base, t), TILE);
       }
       gl_dft_lazy<RL, INV>(x);
-      const int64_t lane = lane0 + c;
-      if (lane >= (int64_t)a.lanes) continue;
-      uint64_t *dst = out + lane * a.out_ls;
+      const uint32_t lane = lane0 + c;
+      if (lane >= a.lanes) continue;
+      uint64_t *dst = out + (uint64_t)a.out_ls * lane;
       if constexpr (GT) {
         // Rows and column batches only: no pass twiddle in this form.
         // k = k1 + R1 * ((k2 * E2 + t * E3) mod S1)
         const int kbase = (k2 * GTC::E2) % S1;
-        dst += (int64_t)k1 * a.out_is;
+        dst += (uint64_t)a.out_is * k1;
         const int64_t kstride = (int64_t)R1 * a.out_is;
         const bool mul = (a.flags & GL_PF_OUT_MUL) != 0;
         const uint64_t *mb = mul ? a.mul + by * a.mul_bs + bz * a.mul_bs2 : nullptr;
@@ -309,13 +314,13 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
           gl_st_out(a, dst + (int64_t)kk * kstride, v);
         }
       } else {
-        const int kbase = k1 + R1 * k2;  // output index of t: kbase + SL*t
-        dst += (int64_t)kbase * a.out_is;
+        const uint32_t kbase = k1 + R1 * k2;  // output index of t: kbase + SL*t
+        dst += (uint64_t)a.out_is * kbase;
         const int64_t kstep = (int64_t)SL * a.out_is;
         if (tw_steps) {
           // tw(col, kbase + SL*t) = tw(col, kbase) * omega_n^(col*SL*t).
-          const uint64_t col = (uint64_t)lane / a.tw_lane_div + a.tw_col0;
-          const uint64_t first = gl_tw2m(a.tw_lo, a.tw_hi, col * (uint64_t)kbase);
+          const uint64_t col = column(lane) + a.tw_col0;
+          const uint64_t first = gl_tw2m(a.tw_lo, a.tw_hi, col * kbase);
 #pragma unroll
           for (int t = 0; t < RL; t++) {
             const uint64_t tw =
@@ -323,7 +328,7 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
             gl_st_out(a, dst + t * kstep, gl_mont_mul(x[t], tw));
           }
         } else if (a.flags & GL_PF_PASS_TWIDDLE) {
-          const uint64_t col = (uint64_t)lane / a.tw_lane_div;
+          const uint64_t col = column(lane);
 #pragma unroll
           for (int t = 0; t < RL; t++)
             gl_st_out(a, dst + t * kstep, gl_mont_mul(x[t], gl_pass_tw(a, col, (uint64_t)(kbase + SL * t))));
