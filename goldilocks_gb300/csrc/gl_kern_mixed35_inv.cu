@@ -4,12 +4,14 @@
 #include "gl_kernels_impl.cuh"
 
 static const gl_kernel_entry k_entries[] = {
-    GL_ENTRY3(16, 16, 6, 4, 1024, true),
-    GL_ENTRY3(16, 16, 10, 4, 1024, true),
-    GL_ENTRY3(16, 16, 12, 4, 1024, true),
+    GL_ENTRY3T(16, 16, 6, 4, 1024, 192, 4, true),
+    GL_ENTRY3T(16, 16, 10, 4, 1024, 320, 2, true),
+    // 680 column tiles (8 355 840 points) ran 1 % slower in the second form,
+    // 1 024 row tiles (12 582 912) 5 % faster.
+    GL_ENTRY3T(16, 16, 12, 4, 1024, 384, 2, true, 5),
     GL_ENTRY3(16, 16, 15, 4, 1024, true),
-    GL_ENTRY3(16, 16, 5, 4, 1024, true),
-    GL_ENTRY3(16, 15, 8, 4, 1024, true),
+    GL_ENTRY3T(16, 16, 5, 4, 1024, 160, 5, true),
+    GL_ENTRY3T(16, 15, 8, 4, 1024, 256, 3, true),
     // 320..768 points (lengths up to about 2^19): 256 threads.
     GL_ENTRY3(16, 16, 3, 4, 256, true),
     GL_ENTRY3(16, 10, 4, 4, 256, true),

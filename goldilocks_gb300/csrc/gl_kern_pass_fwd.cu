@@ -4,7 +4,8 @@
 static const gl_kernel_entry k_entries[] = {
     GL_ENTRY3(8, 8, 1, 4, 32, false),       GL_ENTRY3(16, 8, 1, 4, 32, false),
     GL_ENTRY3(16, 16, 1, 4, 64, false),     GL_ENTRY3(8, 8, 8, 4, 256, false),
-    GL_ENTRY3(16, 8, 8, 4, 512, false),     GL_ENTRY3(16, 16, 8, 4, 1024, false),
+    GL_ENTRY3T(16, 8, 8, 4, 512, 256, 4, false),
+    GL_ENTRY3T(16, 16, 8, 4, 1024, 512, 2, false),
     GL_ENTRY3(16, 16, 16, 4, 1024, false),
 };
 

@@ -4,7 +4,8 @@
 static const gl_kernel_entry k_entries[] = {
     GL_ENTRY3(8, 8, 1, 4, 32, true),       GL_ENTRY3(16, 8, 1, 4, 32, true),
     GL_ENTRY3(16, 16, 1, 4, 64, true),     GL_ENTRY3(8, 8, 8, 4, 256, true),
-    GL_ENTRY3(16, 8, 8, 4, 512, true),     GL_ENTRY3(16, 16, 8, 4, 1024, true),
+    GL_ENTRY3T(16, 8, 8, 4, 512, 256, 4, true),
+    GL_ENTRY3T(16, 16, 8, 4, 1024, 512, 2, true),
     GL_ENTRY3(16, 16, 16, 4, 1024, true),
 };
 

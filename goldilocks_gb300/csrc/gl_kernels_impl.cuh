@@ -38,6 +38,28 @@ static void gl_launch_pass3(const gl_pass_args &args, dim3 grid, cudaStream_t st
    gl_launch_pass3<R1, R2, R3, LANES, NT, INV, MINB>, false,                                  \
    (const void *)gl_pass3_kernel<R1, R2, R3, LANES, NT, INV, MINB>}
 
+// Two forms of one pass: NT threads for a launch of up to PER_SM tiles per SM
+// (two), where a tile's own latency counts, and for more tiles NTM threads with
+// MINB CTAs per SM, sized so that the groups of each round fill whole walks of the
+// threads (the 1024-thread 16 x 16 x 8 form idles half its threads in two
+// rounds of three: barrier stalls 5.4 per issued instruction) and one CTA's
+// loads overlap another's arithmetic.  Measured on GB300 (us): 8 transforms of
+// 2^20 124.9 -> 112.7 (2048-point rows), LDE 2^20 x 64 5589 -> 5130; one 2^20
+// (128 tiles) 23.1 -> 29.1, which is why the first form stays.
+template <int R1, int R2, int R3, int LANES, int NT, int NTM, int MINB, bool INV, int PER_SM = 2>
+static void gl_launch_pass3_by_tiles(const gl_pass_args &args, dim3 grid, cudaStream_t stream, bool pdl) {
+  if ((uint64_t)grid.x * grid.y * grid.z > (uint64_t)PER_SM * (unsigned)gl_sm_count())
+    gl_launch_pass3<R1, R2, R3, LANES, NTM, INV, MINB>(args, grid, stream, pdl);
+  else
+    gl_launch_pass3<R1, R2, R3, LANES, NT, INV>(args, grid, stream, pdl);
+}
+
+#define GL_ENTRY3T(R1, R2, R3, LANES, NT, NTM, MINB, INV, ...)                                \
+  {R1 * R2 * R3, R1, R2, R3, LANES, INV, gl_p3_smem_bytes<R1, R2, R3, LANES>(), NT,          \
+   gl_launch_pass3_by_tiles<R1, R2, R3, LANES, NT, NTM, MINB, INV, ##__VA_ARGS__>, false,     \
+   (const void *)gl_pass3_kernel<R1, R2, R3, LANES, NT, INV, 1>, false,                       \
+   (const void *)gl_pass3_kernel<R1, R2, R3, LANES, NTM, INV, MINB>}
+
 // Good-Thomas inner transform (gcd(R2, R3) = 1): for passes without a pass
 // twiddle (rows, column batches); MINB as above.
 #define GL_ENTRY3G(R1, R2, R3, LANES, NT, MINB, INV)                                          \
