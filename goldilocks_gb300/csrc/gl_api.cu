@@ -234,7 +234,7 @@ extern "C" int gl_preload_kernels(void) {
     size_t n = 0;
     const gl_kernel_entry *e = f(&n);
     for (size_t i = 0; i < n; i++)
-      for (const void *fn : {e[i].func, e[i].func_many})
+      for (const void *fn : {e[i].func, e[i].func2})
         if (fn) funcs.push_back(fn);
   }
   funcs.push_back(gl_generic_kernel_fwd());

@@ -48,7 +48,7 @@ struct gl_kernel_entry {
   bool generic = false;  // gl_generic_kernel: radices passed at run time
   const void *func = nullptr;  // the __global__ function (gl_preload_kernels)
   bool gt = false;             // Good-Thomas inner transform: no pass twiddle allowed
-  const void *func_many = nullptr;  // the form for launches of many tiles, if there is one
+  const void *func2 = nullptr;  // a second form the launcher picks by the arguments, if there is one
 };
 
 // Kernel sets compiled in separate translation units (parallel build).

@@ -19,10 +19,10 @@ const gl_kernel_entry *gl_kernels_pass2_fwd(size_t *count) {
 // Passes up to 512 points over interleaved columns (C > 1): 8-32 adjacent
 // columns per CTA read 64-256-byte row pieces and fill a 256-512-thread CTA.
 static const gl_kernel_entry k_col_entries[] = {
-    GL_ENTRY3M(8, 8, 8, 8, 512, 2, false),
-    GL_ENTRY3M(16, 16, 1, 16, 256, 4, false),
-    GL_ENTRY3M(16, 8, 1, 32, 256, 4, false),
-    GL_ENTRY3M(8, 8, 1, 32, 256, 4, false),
+    GL_ENTRY3C(8, 8, 8, 8, 512, 2, false),
+    GL_ENTRY3C(16, 16, 1, 16, 256, 4, false),
+    GL_ENTRY3C(16, 8, 1, 32, 256, 4, false),
+    GL_ENTRY3C(8, 8, 1, 32, 256, 4, false),
 };
 
 const gl_kernel_entry *gl_kernels_cols_fwd(size_t *count) {

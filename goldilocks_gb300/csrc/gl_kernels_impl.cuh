@@ -3,10 +3,11 @@
 #pragma once
 #include "gl_internal.h"
 
-template <int R1, int R2, int R3, int LANES, int NT, bool INV, int MINB = 1, bool GT = false>
+template <int R1, int R2, int R3, int LANES, int NT, bool INV, int MINB = 1, bool GT = false, bool UNI = false>
 static void gl_launch_pass3(const gl_pass_args &args, dim3 grid, cudaStream_t stream, bool pdl) {
-  constexpr size_t smem = gl_p3_smem_bytes<R1, R2, R3, LANES>();
-  auto kern = gl_pass3_kernel<R1, R2, R3, LANES, NT, INV, MINB, GT>;
+  constexpr size_t smem =
+      UNI ? (size_t)gl_uni_layout<R1, R2, R3, LANES>::WORDS * 8 : gl_p3_smem_bytes<R1, R2, R3, LANES>();
+  auto kern = gl_pass3_kernel<R1, R2, R3, LANES, NT, INV, MINB, GT, UNI>;
   static std::atomic<uint64_t> optin{0};
   gl_smem_optin(optin, kern, smem);
   if (!pdl) {
@@ -59,6 +60,23 @@ static void gl_launch_pass3_by_tiles(const gl_pass_args &args, dim3 grid, cudaSt
    gl_launch_pass3_by_tiles<R1, R2, R3, LANES, NT, NTM, MINB, INV, ##__VA_ARGS__>, false,     \
    (const void *)gl_pass3_kernel<R1, R2, R3, LANES, NT, INV, 1>, false,                       \
    (const void *)gl_pass3_kernel<R1, R2, R3, LANES, NTM, INV, MINB>}
+
+// The uniform form (gl_block3's UNI) where it applies: a pass twiddle from the
+// two-level table, and a number of interleaved columns that is a multiple of
+// the lanes.
+template <int R1, int R2, int R3, int LANES, int NT, int MINB, bool INV>
+static void gl_launch_pass3_cols(const gl_pass_args &args, dim3 grid, cudaStream_t stream, bool pdl) {
+  const bool uniform = (args.flags & (GL_PF_PASS_TWIDDLE | GL_PF_TW_TABLE)) == GL_PF_PASS_TWIDDLE &&
+                       args.tw_lane_div % LANES == 0;
+  if (uniform) gl_launch_pass3<R1, R2, R3, LANES, NT, INV, MINB, false, true>(args, grid, stream, pdl);
+  else gl_launch_pass3<R1, R2, R3, LANES, NT, INV, MINB>(args, grid, stream, pdl);
+}
+
+#define GL_ENTRY3C(R1, R2, R3, LANES, NT, MINB, INV)                                          \
+  {R1 * R2 * R3, R1, R2, R3, LANES, INV, gl_p3_smem_bytes<R1, R2, R3, LANES>(), NT,          \
+   gl_launch_pass3_cols<R1, R2, R3, LANES, NT, MINB, INV>, false,                             \
+   (const void *)gl_pass3_kernel<R1, R2, R3, LANES, NT, INV, MINB>, false,                    \
+   (const void *)gl_pass3_kernel<R1, R2, R3, LANES, NT, INV, MINB, false, true>}
 
 // Good-Thomas inner transform (gcd(R2, R3) = 1): for passes without a pass
 // twiddle (rows, column batches); MINB as above.

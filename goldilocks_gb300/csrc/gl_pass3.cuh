@@ -77,6 +77,24 @@ struct gl_p3_layout {
   static constexpr int WORDS = STEP + NSTEP;
 };
 
+// The tables of the uniform form (gl_block3's UNI), words after the tile:
+//   T2   omega_(R2 R3)^(d3*k2) * omega_n^(col*R1*k2) at [k2*R3 + d3] (three rounds)
+//   PT   the rest of the pass twiddle at [t*R1 + k1]: omega_n^(col*(k1 + SL*t))
+//   IG   the input factor's step g^(S1*itw_jmul*t), t < R1
+//   IB   the input factor's base g^(j*itw_jmul + col), j < S1
+//   T1   the round-1 twiddles times the base: tw_m[g*t] * IB[g] at [t*S1 + g]
+template <int R1, int R2, int R3, int LANES>
+struct gl_uni_layout : gl_p3_layout<R1, R2, R3, LANES> {
+  using B = gl_p3_layout<R1, R2, R3, LANES>;
+  static constexpr int NPT = B::NR == 3 ? R1 * B::RL : B::M;
+  static constexpr int T2 = B::TILE;
+  static constexpr int PT = T2 + (B::NR == 3 ? B::S1 : 0);
+  static constexpr int IG = PT + NPT;
+  static constexpr int IB = IG + R1;
+  static constexpr int T1 = IB + B::S1;
+  static constexpr int WORDS = T1 + B::M;
+};
+
 template <int R1, int R2, int R3, int LANES>
 constexpr size_t gl_p3_smem_bytes() {
   return (size_t)gl_p3_layout<R1, R2, R3, LANES>::WORDS * 8;
@@ -108,10 +126,20 @@ struct gl_gt_consts {
 // One CTA's work: tile (bx, by, bz) of the pass described by `a`, with NT
 // threads and the dynamic shared memory `sm`.  Called by gl_pass3_kernel
 // (tile = blockIdx) and by the persistent batch kernel (tile from its queue).
-template <int R1, int R2, int R3, int LANES, int NT, bool INV, bool GT = false>
+//
+// UNI: a pass with a pass twiddle over interleaved columns whose number is a
+// multiple of LANES, so that the lanes of a tile have one column index: the
+// pass twiddle and the coset factor are tables of the tile.  Each element then
+// takes one product for the pass twiddle (its factor in k2 rides on the round-2
+// twiddle) where a base and a step per lane take two, and the coset factor
+// g^(j*itw_jmul + col), j = g + S1*t, splits into a step in t on the load and
+// a base that rides on the round-1 twiddle, where two table loads, an index
+// computation and two products an element took a quarter of the instructions.
+template <int R1, int R2, int R3, int LANES, int NT, bool INV, bool GT = false, bool UNI = false>
 __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int64_t by,
                                           int64_t bz, uint64_t *sm) {
   using L = gl_p3_layout<R1, R2, R3, LANES>;
+  using U = gl_uni_layout<R1, R2, R3, LANES>;
   using GTC = gl_gt_consts<R2, R3>;
   constexpr int M = L::M;
   constexpr int S1 = R2 * R3;
@@ -132,11 +160,11 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   // launch) and this pass's loads.
   constexpr int SL = L::NR == 3 ? R1 * R2 : R1;  // output stride of the last digit
   const bool tw_steps = (a.flags & (GL_PF_PASS_TWIDDLE | GL_PF_TW_TABLE)) == GL_PF_PASS_TWIDDLE;
-  if constexpr (L::NR == 3 && !GT) {
+  if constexpr (L::NR == 3 && !GT && !UNI) {
     for (int i = threadIdx.x; i < S1; i += NT)
       gl_sm_st(a, sm, L::T2 + i, L::WORDS, __ldg(a.tw_r2 + R1 * (i % R3) * (i / R3)));
   }
-  if constexpr (L::NR > 1) {
+  if constexpr (L::NR > 1 && !UNI) {
     if (tw_steps) {
       for (uint32_t i = threadIdx.x; i < L::NSTEP; i += NT) {
         const uint32_t c = i / L::SS, t = i % L::SS;
@@ -163,8 +191,43 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   // Every lane and index of the tile is there (uniform over the CTA).
   const bool whole = lane0 + LANES <= a.lanes && lane0 + LANES > lane0 && a.in_limit >= (uint32_t)M;
 
+  const bool in_twiddle = (a.flags & GL_PF_IN_TWIDDLE) != 0;
+  // The uniform form's tables, staged behind the data loads of round 1.
+  [[maybe_unused]] auto stage_uniform = [&]() {
+    const uint64_t col = column(lane0) + a.tw_col0;
+    if constexpr (L::NR == 3) {
+      for (uint32_t i = threadIdx.x; i < S1; i += NT) {
+        const uint32_t k2 = i / R3, d3 = i % R3;
+        uint64_t v = gl_tw2m(a.tw_lo, a.tw_hi, col * (R1 * k2));
+        if (a.tw_unscale) v = gl_mont_mul(v, a.tw_unscale);
+        gl_sm_st(a, sm, U::T2 + i, U::WORDS, gl_mont_mul(v, __ldg(a.tw_r2 + R1 * d3 * k2)));
+      }
+    }
+    for (uint32_t i = threadIdx.x; i < U::NPT; i += NT)  // k = k1 + SL*t; two rounds: k = i
+      gl_sm_st(a, sm, U::PT + i, U::WORDS, gl_tw2m(a.tw_lo, a.tw_hi, col * (L::NR == 3 ? i % R1 + SL * (i / R1) : i)));
+    if (in_twiddle) {
+      // Indices at or past in_limit load as zero and lie outside the tables:
+      // their factor is any word.
+      const uint32_t icol = column(lane0);
+      for (uint32_t i = threadIdx.x; i < R1; i += NT)
+        gl_sm_st(a, sm, U::IG + i, U::WORDS,
+                 S1 * i < a.in_limit ? gl_tw2m(a.itw_lo, a.itw_hi, (uint64_t)(S1 * i) * a.itw_jmul) : 0);
+      for (uint32_t i = threadIdx.x; i < S1; i += NT)
+        gl_sm_st(a, sm, U::IB + i, U::WORDS,
+                 i < a.in_limit ? gl_tw2m(a.itw_lo, a.itw_hi, i * a.itw_jmul + icol) : 0);
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < (uint32_t)M; i += NT) {
+        const uint32_t g = i % S1, t = i / S1;
+        gl_sm_st(a, sm, U::T1 + i, U::WORDS,
+                 gl_mont_mul(__ldg(a.tw_m + g * t), gl_sm_ld(a, sm, U::IB + g, U::WORDS)));
+      }
+    }
+    __syncthreads();
+  };
+
   // ------------------------------------------------------------- round 1
   {
+    static_assert(!UNI || (!GT && L::NR > 1 && LANES * (M / R1) == NT), "one round-1 group per thread");
     constexpr uint32_t G = M / R1;  // groups per lane: jB = (d2, d3)
     GL_ROUND(idx, LANES * G) {
       uint32_t c, g;
@@ -185,7 +248,13 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
           x[t] = (live && j < a.in_limit) ? gl_ld_in(a, src + t * step, load_cg) : 0;
         }
       }
-      if (a.flags & GL_PF_IN_TWIDDLE) {
+      if constexpr (UNI) {
+        stage_uniform();
+        if (in_twiddle) {
+#pragma unroll
+          for (int t = 1; t < R1; t++) x[t] = gl_mont_mul(x[t], gl_sm_ld(a, sm, U::IG + t, U::WORDS));
+        }
+      } else if (in_twiddle) {
         const uint32_t col = column(lane);
 #pragma unroll
         for (int t = 0; t < R1; t++) {
@@ -219,6 +288,12 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
         }
       } else {
         const uint32_t base = L::word(c, g);
+        if (UNI && in_twiddle) {
+#pragma unroll
+          for (int t = 0; t < R1; t++)
+            gl_sm_st(a, sm, L::at(base, S1 * t), TILE, gl_mont_mul(x[t], gl_sm_ld(a, sm, U::T1 + S1 * t + g, U::WORDS)));
+          continue;
+        }
 #pragma unroll
         for (int t = 0; t < R1; t++) {
           uint64_t v = x[t];
@@ -254,14 +329,14 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
         for (int t = 0; t < R2; t++) gl_sm_st(a, sm, pos[t], TILE, x[t]);
       } else {
         const uint32_t base = L::word(c, k1 * S1 + d3);
-        const uint32_t tw = L::T2 + d3;
+        const uint32_t tw = (UNI ? (int)U::T2 : (int)L::T2) + d3;
 #pragma unroll
         for (int t = 0; t < R2; t++) x[t] = gl_sm_ld(a, sm, L::at(base, R3 * t), TILE);
         gl_dft_lazy<R2, INV>(x);
 #pragma unroll
         for (int t = 0; t < R2; t++) {
           uint64_t v = x[t];
-          if (t > 0) v = gl_mont_mul(v, gl_sm_ld(a, sm, tw + R3 * t, L::WORDS));
+          if (t > 0) v = gl_mont_mul(v, gl_sm_ld(a, sm, tw + R3 * t, UNI ? (int)U::WORDS : (int)L::WORDS));
           gl_sm_st(a, sm, L::at(base, R3 * t), TILE, v);
         }
       }
@@ -317,7 +392,11 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
         const uint32_t kbase = k1 + R1 * k2;  // output index of t: kbase + SL*t
         dst += (uint64_t)a.out_is * kbase;
         const int64_t kstep = (int64_t)SL * a.out_is;
-        if (tw_steps) {
+        if constexpr (UNI) {
+#pragma unroll
+          for (int t = 0; t < RL; t++)
+            gl_st_out(a, dst + t * kstep, gl_mont_mul(x[t], gl_sm_ld(a, sm, U::PT + R1 * t + k1, U::WORDS)));
+        } else if (tw_steps) {
           // tw(col, kbase + SL*t) = tw(col, kbase) * omega_n^(col*SL*t).
           const uint64_t col = column(lane) + a.tw_col0;
           const uint64_t first = gl_tw2m(a.tw_lo, a.tw_hi, col * kbase);
@@ -346,8 +425,8 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   }
 }
 
-template <int R1, int R2, int R3, int LANES, int NT, bool INV, int MINB = 1, bool GT = false>
+template <int R1, int R2, int R3, int LANES, int NT, bool INV, int MINB = 1, bool GT = false, bool UNI = false>
 __global__ void __launch_bounds__(NT, MINB) gl_pass3_kernel(const gl_pass_args a) {
   extern __shared__ uint64_t sm[];
-  gl_block3<R1, R2, R3, LANES, NT, INV, GT>(a, blockIdx.x, blockIdx.y, blockIdx.z, sm);
+  gl_block3<R1, R2, R3, LANES, NT, INV, GT, UNI>(a, blockIdx.x, blockIdx.y, blockIdx.z, sm);
 }
