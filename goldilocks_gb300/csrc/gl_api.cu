@@ -951,6 +951,24 @@ extern "C" int gl_debug_check_status(uint32_t *flags) {
 #endif
 }
 
+// Whether the first pass of a call may be launched programmatically, too: the
+// pass waits (gl_pdl_wait) for the kernel before it in the stream, whoever's it
+// is, before it reads or writes anything but its plan's tables, which were
+// complete before the plan was handed out.  Back to back calls then overlap
+// one's launch with the other's last wave.  Measured on GB300, calls back to
+// back (us): 1 024 points 6.2 -> 3.3, 2^13 10.2 -> 6.4, 2^16 10.3 -> 8.0, 2^20
+// 22.6 -> 18.8, 1 052 672 58.1 -> 45.5, 2^16 x 64 columns 47.2 -> 44.4,
+// 16 711 680 313.9 -> 305.7.  A launch of many waves gains nothing and the LDE's
+// (107 tiles an SM) ran 0.6 % slower, so those start plainly.  So does a call
+// inside a stream capture, where it would add a programmatic edge to a graph of
+// the caller's.
+bool gl_first_pass_pdl(cudaStream_t stream, uint64_t tiles) {
+  if (tiles > 16ull * (unsigned)gl_sm_count()) return false;
+  if (stream == nullptr || stream == cudaStreamLegacy) return true;  // never captured
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
 // Queue the transform of a strided batch on `stream`.  Element j of column c
 // of batch item b is at base[b*bs + j*C + c] (C = 1, bs = n: contiguous
 // transforms; C = cols, B = 1: the columns of a row-major matrix).  `src` and
@@ -987,6 +1005,9 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
   if (st != GL_OK) return st;
   const int d = inv ? 1 : 0;
   const bool coset = lo->itw_lo != nullptr;
+  // With factors (om) the last pass reads them through the non-coherent path,
+  // so no pass may start before the kernel that wrote them has finished.
+  auto pdl = [&](uint64_t tiles) { return !om && gl_first_pass_pdl(stream, tiles); };
   auto base_args = [&]() {
     gl_pass_args a{};
     a.in_limit = lo->in_limit;
@@ -1012,13 +1033,14 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
       if (coset) { a.itw_jmul = 1; a.tw_lane_div = 0xffffffffu; }
       if (om) { a.flags |= mul_flags; a.mul_ls = mul_item; }  // lane = batch item
       const uint64_t per = (uint64_t)k->lanes * 0x7fffffffull;
+      const bool early = pdl(gl_tiles(B, k));
       for (uint64_t off = 0; off < B; off += per) {
         const uint64_t c = std::min(per, B - off);
         a.in = src + off * bs; a.out = dst + off * bs;
         if (om) a.mul = om->factors + off * mul_item;
         a.lanes = (uint32_t)c;
         GL_DBG_EXTENTS(a, (c - 1) * bs + n, (c - 1) * bs + out_ext);
-        gl_launch(k, 0, a, dim3((unsigned)((c + k->lanes - 1) / k->lanes)), c * n, stream);
+        gl_launch(k, 0, a, dim3((unsigned)((c + k->lanes - 1) / k->lanes)), c * n, stream, early);
       }
     } else {
       // Lanes are the C interleaved columns; batch items on grid.y.
@@ -1027,12 +1049,13 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
       a.flags |= GL_PF_LOAD_LANE_FAST | GL_PF_STORE_LANE_FAST;
       if (coset) { a.itw_jmul = 1; a.tw_lane_div = 0xffffffffu; }
       a.lanes = (uint32_t)C;
+      const bool early = pdl(gl_tiles(C, k) * B);
       for (uint64_t off = 0; off < B; off += kMaxGridYZ) {
         const uint64_t c = std::min(kMaxGridYZ, B - off);
         a.in = src + off * bs; a.out = dst + off * bs;
         GL_DBG_EXTENTS(a, (c - 1) * bs + n * C, (c - 1) * bs + out_ext);
         gl_launch(k, 0, a, dim3((unsigned)((C + k->lanes - 1) / k->lanes), (unsigned)c),
-               c * n * C, stream);
+               c * n * C, stream, early);
       }
     }
     return gl_cuda_status(cudaGetLastError());
@@ -1040,8 +1063,6 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
   if (pl->kind == 3) {
     // Three passes, n = n1*n2*n3, j = n2 n3 j1 + n3 j2 + j3,
     // k = k1 + n1 k2 + n1 n2 k3:
-    // Every pass after the first of the call is launched for programmatic
-    // dependent launch: its predecessor in the stream is a pass of this call.
     //   A  n1-point over j1, times omega_n^(j23 k1)           src -> scratch
     //   B  per k1: n2-point over j2, times omega_(n2 n3)^(j3 k2)  in place
     //   C  per (k1, k2): n3-point over j3, stored at k         scratch -> dst
@@ -1068,7 +1089,7 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
       GL_DBG_EXTENTS(a, n * C, n * C);
       const uint64_t ta = gl_tiles(n23 * C, ka);
       if (ta > 0x7fffffffull) return GL_ERR_INVALID;
-      gl_launch(ka, 1, a, dim3((unsigned)ta), n * C, stream, b > 0);
+      gl_launch(ka, 1, a, dim3((unsigned)ta), n * C, stream, b > 0 || pdl(ta));
       gl_pass_args bb = base_args();
       bb.in_limit = 0xffffffffu;
       bb.in = s1; bb.out = s1;
@@ -1111,8 +1132,7 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
     }
     return gl_cuda_status(cudaGetLastError());
   }
-  // Four-step: n = n1*n2, j = n2*j1 + j2, k = k1 + n1*k2.  Every pass after
-  // the first of the call is launched for programmatic dependent launch.
+  // Four-step: n = n1*n2, j = n2*j1 + j2, k = k1 + n1*k2.
   const uint64_t n1 = pl->n1, n2 = pl->n2;
   const auto &ks = C > 1 ? pl->k4 : pl->k;  // interleaved columns: four-lane kernels
   const gl_kernel_entry *kc = ks[0][d], *kr = ks[1][d];
@@ -1141,7 +1161,7 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
     const uint64_t lanes1 = n2 * C;
     if (gl_tiles(lanes1, kc) > 0x7fffffffull) return GL_ERR_INVALID;
     gl_launch(kc, 1, a, dim3((unsigned)gl_tiles(lanes1, kc), (unsigned)cb),
-              cb * n * C, stream, off > 0);
+              cb * n * C, stream, off > 0 || pdl(gl_tiles(lanes1, kc) * cb));
     // ROW: n2-point transforms along j2 for every (k1, c); transposed store.
     gl_pass_args b = base_args();
     b.in_limit = 0xffffffffu;  // zero padding applies to the first pass only

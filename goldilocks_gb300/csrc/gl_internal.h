@@ -32,8 +32,9 @@ cudaError_t gl_malloc_async(void **p, size_t bytes, cudaStream_t stream);
 cudaMemPool_t gl_mempool();
 
 // pdl: launch with programmatic stream serialization (the kernel may start
-// while the previous kernel of the stream finishes; see gl_pdl_wait).  Only
-// for a pass whose predecessor in the stream is a pass of the same call.
+// while the previous kernel of the stream finishes; see gl_pdl_wait).  Not
+// where an earlier operation of the stream may still be writing the tables the
+// pass stages before its wait.
 typedef void (*gl_launch_fn)(const gl_pass_args &args, dim3 grid, cudaStream_t stream, bool pdl);
 
 // One compiled instance of a pass kernel: gl_pass3_kernel (radices r1 x r2 x
@@ -180,6 +181,9 @@ void gl_launch(const gl_kernel_entry *k, int role, const gl_pass_args &a, dim3 g
 int gl_cuda_status(cudaError_t e);
 void gl_init_mempool_once();
 int gl_sm_count();  // multiprocessors of the current device
+// Whether the first kernel of a call, `tiles` CTAs on `stream`, is launched with
+// `pdl`.
+bool gl_first_pass_pdl(cudaStream_t stream, uint64_t tiles);
 // Scratch words gl_coset_lde takes beside the n x cols coefficients.
 uint64_t gl_lde_scratch_words(gl_plan *pn, gl_plan *pm, uint64_t n, uint64_t cols, uint32_t blowup);
 void gl_pipeline_release_blocks();  // idle device blocks cached by gl_host_pipeline (gl_pipeline.cu)

@@ -31,10 +31,12 @@ enum : uint32_t {
 
 // Programmatic dependent launch (griddepcontrol, sm_90 and later).  A pass
 // launched with programmatic stream serialization may start once every CTA
-// of the previous kernel in its stream has started; it waits in gl_pdl_wait
-// -- until that kernel has finished and its writes are visible -- before it
-// reads data or writes global memory.  Without that launch attribute both are
-// no-ops.
+// of the previous kernel in its stream has started (a pass of this library) or
+// finished (any other kernel); it waits in gl_pdl_wait -- until that kernel has
+// finished and its writes are visible -- before it reads data or writes global
+// memory.  What a kernel that may still be running when this one starts can
+// write is not read through the non-coherent path (__ldg).  Without that launch
+// attribute both are no-ops.
 __device__ __forceinline__ void gl_pdl_launch_dependents() {
 #if defined(__CUDA_ARCH__)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -140,6 +142,10 @@ __device__ __forceinline__ uint64_t gl_tw2m(const uint64_t *lo, const uint64_t *
 // Pointwise factor on the final store; `mb` is mul + by*mul_bs + bz*mul_bs2.
 __device__ __forceinline__ uint64_t gl_out_mul(const gl_pass_args &a, const uint64_t *mb,
                                                int64_t lane, int64_t k, uint64_t v) {
+  // The factors are the caller's: a call with factors starts no pass before
+  // the kernel ahead of it has finished (gl_enqueue_transform), so they may take
+  // the non-coherent path, whose loads run ahead of the stores (a plain load's
+  // do not: convolution at 2^22 152.8 against 146.0 us).
   v = gl_mul(v, __ldg(mb + lane * a.mul_ls + k * a.out_is));
   return (a.flags & GL_PF_OUT_MUL_MONT) ? gl_shl<128>(v) : v;  // 2^128 = 2^-64
 }

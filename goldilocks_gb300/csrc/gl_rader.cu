@@ -43,11 +43,29 @@ int upload(gl_dev_tables &t, const std::vector<T> &h, T **dst) {
   return gl_table_upload(t, h.data(), h.size() * sizeof(T), (void **)dst);
 }
 
+// Launched with programmatic stream serialization: every kernel of a Rader step
+// waits for the one before it in the stream before it touches data.
+template <typename... P, typename... A>
+int launch(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t stream, bool pdl, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return gl_cuda_status(cudaLaunchKernelEx(&cfg, kern, (P)args...));
+}
+
 }  // namespace
 
 // Row r of `A` (r < q - 1) is row gpow[r] of `src`; row 0 of `src` goes to x0.
 __global__ void gl_rader_gather_kernel(const uint64_t *src, uint64_t *A, uint64_t *x0,
                                        const uint32_t *gpow, uint64_t L, uint32_t q) {
+  gl_pdl_launch_dependents();
+  gl_pdl_wait();
   const uint64_t total = (uint64_t)q * L;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -60,6 +78,8 @@ __global__ void gl_rader_gather_kernel(const uint64_t *src, uint64_t *A, uint64_
 // X0 = x0 + A[0] (the sum of all inputs but x0), then A[p] *= bhat[p].
 __global__ void gl_rader_pointwise_kernel(uint64_t *A, const uint64_t *x0, uint64_t *X0,
                                           const uint64_t *bhat, uint64_t L, uint32_t rows) {
+  gl_pdl_launch_dependents();
+  gl_pdl_wait();
   const uint64_t total = (uint64_t)rows * L;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -75,6 +95,8 @@ __global__ void gl_rader_pointwise_kernel(uint64_t *A, const uint64_t *x0, uint6
 __global__ void gl_rader_scatter_kernel(const uint64_t *conv, const uint64_t *x0, const uint64_t *X0,
                                         uint64_t *Y, const uint32_t *gneg, const uint64_t *tw_lo,
                                         const uint64_t *tw_hi, uint64_t C, uint64_t L, uint32_t q) {
+  gl_pdl_launch_dependents();
+  gl_pdl_wait();
   const uint64_t total = (uint64_t)q * L;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -102,6 +124,8 @@ __global__ void __launch_bounds__(256) gl_rader_scatter_tiled_kernel(
     const uint64_t *conv, const uint64_t *x0, const uint64_t *X0, uint64_t *Y, const uint32_t *kpos,
     const uint64_t *tw_lo, const uint64_t *tw_hi, uint64_t C, uint64_t L, uint32_t q) {
   __shared__ uint64_t tile[32][33];
+  gl_pdl_launch_dependents();
+  gl_pdl_wait();
   const uint64_t l0 = (uint64_t)blockIdx.x * 32, k0 = (uint64_t)blockIdx.y * 32;
   for (int i = threadIdx.y; i < 32; i += 8) {
     const uint64_t k1 = k0 + i, l = l0 + threadIdx.x;
@@ -183,24 +207,22 @@ int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C
   for (uint64_t b = 0; b < B; b++) {
     const uint64_t *in = src + b * bs;
     uint64_t *out = dst + b * bs;
-    gl_rader_gather_kernel<<<grid_for(q * L), 256, 0, stream>>>(in, A, x0, t->rader_gpow, L, (uint32_t)q);
-    if ((st = gl_cuda_status(cudaGetLastError())) != GL_OK) return st;
+    if ((st = launch(gl_rader_gather_kernel, grid_for(q * L), 256, stream, b > 0 || gl_first_pass_pdl(stream, 0), in,
+                     A, x0, t->rader_gpow, L, q)) != GL_OK)
+      return st;
     if ((st = gl_enqueue_transform(pl->pq, A, A, L, 1, r * L, false, sub, stream)) != GL_OK) return st;
-    gl_rader_pointwise_kernel<<<grid_for(r * L), 256, 0, stream>>>(A, x0, X0, t->rader_bhat[d], L,
-                                                                   (uint32_t)r);
-    if ((st = gl_cuda_status(cudaGetLastError())) != GL_OK) return st;
+    if ((st = launch(gl_rader_pointwise_kernel, grid_for(r * L), 256, stream, true, A, x0, X0, t->rader_bhat[d], L,
+                     r)) != GL_OK)
+      return st;
     if ((st = gl_enqueue_transform(pl->pq, A, A, L, 1, r * L, true, sub, stream)) != GL_OK) return st;
     uint64_t *target = m > 1 ? Y : out;
-    if (C < 8) {
-      const dim3 grid((unsigned)((L + 31) / 32), (unsigned)((q + 31) / 32));
-      gl_rader_scatter_tiled_kernel<<<grid, dim3(32, 8), 0, stream>>>(
-          A, x0, X0, target, t->rader_kpos, t->rader_tw_lo[d], t->rader_tw_hi[d], C, L, (uint32_t)q);
-    } else {
-      gl_rader_scatter_kernel<<<grid_for(q * L), 256, 0, stream>>>(A, x0, X0, target, t->rader_gneg,
-                                                                   t->rader_tw_lo[d], t->rader_tw_hi[d],
-                                                                   C, L, (uint32_t)q);
-    }
-    if ((st = gl_cuda_status(cudaGetLastError())) != GL_OK) return st;
+    if (C < 8)
+      st = launch(gl_rader_scatter_tiled_kernel, dim3((unsigned)((L + 31) / 32), (unsigned)((q + 31) / 32)),
+                  dim3(32, 8), stream, true, A, x0, X0, target, t->rader_kpos, t->rader_tw_lo[d], t->rader_tw_hi[d], C, L, q);
+    else
+      st = launch(gl_rader_scatter_kernel, grid_for(q * L), 256, stream, true, A, x0, X0, target, t->rader_gneg,
+                  t->rader_tw_lo[d], t->rader_tw_hi[d], C, L, q);
+    if (st != GL_OK) return st;
     if (m > 1 && (st = gl_enqueue_transform(pl->pm, Y, out, q * C, 1, n * C, inv, sub, stream)) != GL_OK)
       return st;
   }
