@@ -14,6 +14,7 @@ the tensor's current stream).  Unsupported sizes raise ValueError with the
 reference's panic message.
 """
 import ctypes
+import sys
 
 import numpy as np
 
@@ -45,18 +46,17 @@ def _buffer(values):
         if not values.flags.c_contiguous or not values.flags.writeable:
             raise ValueError("host values must be C-contiguous and writeable")
         return values.ctypes.data, values.size, L.GL_MEM_HOST, None
-    try:
-        import torch
-    except ImportError:  # pragma: no cover
-        torch = None
+    torch = sys.modules.get("torch")  # a tensor's module is loaded
     if torch is not None and isinstance(values, torch.Tensor):
         if not values.is_cuda:
             raise ValueError("torch tensors must live on a CUDA device (use numpy for host data)")
-        if values.element_size() != 8 or values.dtype.is_floating_point:
+        if values.dtype is not torch.int64 and (values.element_size() != 8 or values.dtype.is_floating_point):
             raise TypeError("device values must be a 64-bit integer tensor")
         if not values.is_contiguous():
             raise ValueError("device values must be contiguous")
-        stream = torch.cuda.current_stream(values.device).cuda_stream
+        # The stream's handle without the torch.cuda.Stream object around it:
+        # the object was a third of a short call's host time.
+        stream = torch._C._cuda_getCurrentRawStream(values.get_device())
         return values.data_ptr(), values.numel(), L.GL_MEM_DEVICE, stream
     raise TypeError("values must be a numpy uint64 array or a CUDA torch tensor")
 
