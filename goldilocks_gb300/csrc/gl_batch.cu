@@ -362,6 +362,41 @@ struct bucket_graph {
 std::mutex g_graph_mu;
 std::map<std::vector<std::pair<uint64_t, int>>, std::unique_ptr<bucket_graph>> g_graphs;
 
+// Streams a bucket graph is captured on: s[0] begins the capture, the others
+// fork from it and join it again.
+constexpr int kBranches = 4;
+struct branches {
+  cudaStream_t s[kBranches] = {};
+  cudaEvent_t ev[kBranches] = {};
+  cudaError_t create() {
+    for (int i = 0; i < kBranches; i++) {
+      cudaError_t e = cudaStreamCreateWithFlags(&s[i], cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  }
+  cudaError_t fork() {
+    cudaError_t e = cudaEventRecord(ev[0], s[0]);
+    for (int i = 1; i < kBranches && e == cudaSuccess; i++) e = cudaStreamWaitEvent(s[i], ev[0], 0);
+    return e;
+  }
+  cudaError_t join() {
+    cudaError_t e = cudaSuccess;
+    for (int i = 1; i < kBranches && e == cudaSuccess; i++) {
+      e = cudaEventRecord(ev[i], s[i]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(s[0], ev[i], 0);
+    }
+    return e;
+  }
+  ~branches() {
+    for (int i = 0; i < kBranches; i++) {
+      if (ev[i]) cudaEventDestroy(ev[i]);
+      if (s[i]) cudaStreamDestroy(s[i]);
+    }
+  }
+};
+
 int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_plan> &pp,
                 cudaStream_t stream) {
   // Group by (len, dir); order within a bucket = input order.
@@ -416,14 +451,31 @@ int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_pla
       return gl_cuda_status(e);
     }
     uint64_t **dt = (uint64_t **)g->tables;
-    cudaStream_t cap;
-    if ((e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking)) != cudaSuccess) return gl_cuda_status(e);
+    // The buckets are independent: they go to kBranches branches of the graph,
+    // each bucket to the branch with the fewest elements so far, the largest
+    // first, so that one kernel's last wave runs beside another's first (in
+    // one chain the 28 kernels of the 1 024-polynomial batch drained one after
+    // another: 975 against 935 us a batch on GB300).
+    branches br;
+    if ((e = br.create()) != cudaSuccess) return gl_cuda_status(e);
+    cudaStream_t cap = br.s[0];
     cudaGraph_t graph;
+    std::vector<std::pair<size_t, size_t>> runs;  // items [first, end) of a bucket
+    for (size_t j = 0, j1; j < nitems; j = j1) {
+      for (j1 = j; j1 < nitems && sig[j1] == sig[j];) j1++;
+      runs.push_back({j, j1});
+    }
+    auto work = [&](const std::pair<size_t, size_t> &r) { return sig[r.first].first * (r.second - r.first); };
+    std::stable_sort(runs.begin(), runs.end(), [&](const auto &x, const auto &y) { return work(x) > work(y); });
+    uint64_t load[kBranches] = {};
     e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-    size_t j = 0;
-    while (e == cudaSuccess && j < nitems) {
-      size_t j1 = j;
-      while (j1 < nitems && sig[j1] == sig[j]) j1++;
+    if (e == cudaSuccess) e = br.fork();
+    for (const auto &r : runs) {
+      if (e != cudaSuccess) break;
+      const size_t j = r.first, j1 = r.second;
+      const int to = (int)(std::min_element(load, load + kBranches) - load);
+      load[to] += work(r);
+      const cudaStream_t on = br.s[to];
       const poly_plan &p = pp[order[j]];
       const gl_plan *pl = p.pl;
       const int d = p.inv ? 1 : 0;
@@ -433,27 +485,29 @@ int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_pla
         full.flags |= GL_PF_PTR_TABLE;
         full.in_ptrs = (const uint64_t *const *)(dt + j);
         full.out_ptrs = (uint64_t *const *)(dt + j);
-        gl_launch(pl->k[0][d], 0, full, dim3(1, (unsigned)(j1 - j)), pl->size * (j1 - j), cap);
+        // One polynomial per CTA: the one-transform kernel where there is one
+        // (the others' lanes but one are dead here).
+        const gl_kernel_entry *k = pl->k1[d] ? pl->k1[d] : pl->k[0][d];
+        gl_launch(k, 0, full, dim3(1, (unsigned)(j1 - j)), pl->size * (j1 - j), on);
       } else {
         const size_t base_sc = nitems;
         col.flags |= GL_PF_PTR_TABLE;
         col.in_ptrs = (const uint64_t *const *)(dt + j);
         col.out_ptrs = (uint64_t *const *)(dt + base_sc + j);
         gl_launch(pl->k[0][d], 1, col, dim3((unsigned)gl_tiles(pl->n2, pl->k[0][d]), (unsigned)(j1 - j)),
-                  pl->size * (j1 - j), cap);
+                  pl->size * (j1 - j), on);
         row.flags |= GL_PF_PTR_TABLE;
         row.in_ptrs = (const uint64_t *const *)(dt + base_sc + j);
         row.out_ptrs = (uint64_t *const *)(dt + j);
         gl_launch(pl->k[1][d], 2, row, dim3((unsigned)gl_tiles(pl->n1, pl->k[1][d]), (unsigned)(j1 - j)),
-                  pl->size * (j1 - j), cap);
+                  pl->size * (j1 - j), on, true);
       }
-      j = j1;
     }
+    if (e == cudaSuccess) e = br.join();
     cudaError_t e2 = cudaStreamEndCapture(cap, &graph);
     if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, graph, 0);
     if (e2 == cudaSuccess) cudaGraphDestroy(graph);
-    cudaStreamDestroy(cap);
     if (e != cudaSuccess) {
       g_graphs.erase(sig);  // g frees its tables
       return gl_cuda_status(e);
