@@ -612,11 +612,14 @@ __global__ void gl_fill_pass_twiddles(uint64_t *out, const uint64_t *lo, const u
 }
 
 // Full pass-twiddle tables (8 bytes per element and direction; one load and
-// one multiplication per element instead of two loads and two) are built for
-// plans up to this size when GOLDILOCKS_PASS_TWIDDLE=full.  Measured on GB300
-// at 2^24 the two-level table is faster (the column pass is bound by the
-// integer pipe, and the table load sits on its critical path), so it is the
-// default.
+// one multiplication per element instead of two loads and two).  Two-pass plans
+// up to kFullTwiddleDefault points have them (128 KiB per direction at most),
+// for contiguous transforms: many transforms share the table in L2.  Measured
+// on GB300 (us): 1 024 transforms of 4 096 points 45.1 -> 41.1, 256 of 16 384
+// 46.0 -> 41.5; at 2^16 to 2^20 the gain is 1 %, and from 2^22 on the table
+// is read from HBM and the pass is 15 % slower.  GOLDILOCKS_PASS_TWIDDLE=full
+// builds them up to kFullTwiddleMax points, for interleaved columns as well.
+static const uint64_t kFullTwiddleDefault = 1ull << 14;
 static const uint64_t kFullTwiddleMax = 1ull << 26;
 static bool full_twiddles_enabled() {
   static const bool on = [] {
@@ -653,7 +656,7 @@ int gl_plan_tables(gl_plan *pl, gl_dev_tables **out) {
       if (d) t.tw_unscale[d] = gl_to_mont(n % GL_P);
       if (st == GL_OK) st = upload(t, mont_powers(w, GL_TW_SPLIT, scale), &t.tw_lo[d]);
       if (st == GL_OK) st = upload(t, mont_powers(gl_pow(w, GL_TW_SPLIT), hi_count, 1), &t.tw_hi[d]);
-      if (st == GL_OK && n <= kFullTwiddleMax && full_twiddles_enabled()) {
+      if (st == GL_OK && n <= (full_twiddles_enabled() ? kFullTwiddleMax : kFullTwiddleDefault)) {
         cudaStream_t ts = gl_table_stream();
         void *p = nullptr;
         cudaError_t e = gl_malloc_async(&p, n * sizeof(uint64_t), ts);
@@ -1148,7 +1151,7 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
     a.tw_m = a.tw_r2 = t->blk[0][d]; a.tw_lo = t->tw_lo[d]; a.tw_hi = t->tw_hi[d];
     a.tw_unscale = t->tw_unscale[d];
     a.tw_lane_div = (uint32_t)C;
-    if (t->tw_full[d]) {
+    if (t->tw_full[d] && (C == 1 || full_twiddles_enabled())) {
       a.flags |= GL_PF_TW_TABLE;
       a.tw_full = t->tw_full[d];
       a.tw_ld = (int64_t)n2;
