@@ -143,6 +143,18 @@ static bool generic_radices(uint64_t m, int r[3]) {
   return false;
 }
 
+// The compiled four-lane kernel that runs m points in the run-time-radix
+// kernel's place, or nullptr.
+static const gl_kernel_entry *fixed_radix_entry(uint64_t m, bool inv) {
+  size_t cnt = 0;
+  const gl_kernel_entry *e = inv ? gl_kernels_small_inv(&cnt) : gl_kernels_small_fwd(&cnt);
+  if (const gl_kernel_entry *k = find_in(e, cnt, m)) return k;
+  e = inv ? gl_kernels_mixed35_inv(&cnt) : gl_kernels_mixed35_fwd(&cnt);
+  if (const gl_kernel_entry *k = find_in(e, cnt, m)) return k;
+  e = inv ? gl_kernels_mixed17_inv(&cnt) : gl_kernels_mixed17_fwd(&cnt);
+  return find_in(e, cnt, m);
+}
+
 static const gl_kernel_entry *generic_entry(uint64_t m, bool inv) {
   static std::mutex mu;
   static std::map<std::pair<uint64_t, bool>, gl_kernel_entry> cache;
@@ -157,7 +169,11 @@ static const gl_kernel_entry *generic_entry(uint64_t m, bool inv) {
   e.lanes = GL_GEN_LANES; e.inv = inv;
   e.smem = r[1] == 1 ? 0 : (size_t)GL_GEN_LANES * gl_gen_ls((int)m) * sizeof(uint64_t);
   e.threads = GL_GEN_NT;
-  e.launch = inv ? gl_launch_generic_inv : gl_launch_generic_fwd;
+  // Radices are still chosen at run time (and plans rank the size so), but
+  // where a kernel is compiled for the size the launch goes to it.
+  const gl_kernel_entry *fixed = fixed_radix_entry(m, inv);
+  static_assert(GL_GEN_LANES == 4, "the compiled kernels of these sizes have four lanes");
+  e.launch = fixed ? fixed->launch : inv ? gl_launch_generic_inv : gl_launch_generic_fwd;
   e.generic = true;
   return &cache.emplace(key, e).first->second;
 }
@@ -228,7 +244,7 @@ extern "C" int gl_preload_kernels(void) {
   for (table_fn f : {gl_kernels_full_fwd, gl_kernels_full_inv, gl_kernels_full1_fwd, gl_kernels_full1_inv,
                      gl_kernels_gt17_fwd, gl_kernels_gt17_inv,
                      gl_kernels_pass_fwd, gl_kernels_pass_inv,
-                     gl_kernels_mixed35_fwd, gl_kernels_mixed35_inv, gl_kernels_mixed17_fwd,
+                     gl_kernels_small_fwd, gl_kernels_small_inv, gl_kernels_mixed35_fwd, gl_kernels_mixed35_inv, gl_kernels_mixed17_fwd,
                      gl_kernels_mixed17_inv, gl_kernels_pass2_fwd, gl_kernels_pass2_inv, gl_kernels_cols_fwd,
                      gl_kernels_cols_inv}) {
     size_t n = 0;

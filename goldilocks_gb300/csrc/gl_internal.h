@@ -73,6 +73,9 @@ const gl_kernel_entry *gl_kernels_mixed35_fwd(size_t *count);
 const gl_kernel_entry *gl_kernels_mixed35_inv(size_t *count);
 const gl_kernel_entry *gl_kernels_mixed17_fwd(size_t *count);
 const gl_kernel_entry *gl_kernels_mixed17_inv(size_t *count);
+// Four-lane kernels of fixed radices for sizes that plans treat as run-time radices.
+const gl_kernel_entry *gl_kernels_small_fwd(size_t *count);
+const gl_kernel_entry *gl_kernels_small_inv(size_t *count);
 // Passes up to 2048 points with two lanes per CTA and four CTAs per SM.
 const gl_kernel_entry *gl_kernels_pass2_fwd(size_t *count);
 const gl_kernel_entry *gl_kernels_pass2_inv(size_t *count);
