@@ -46,7 +46,13 @@ static void gl_launch_pass3(const gl_pass_args &args, dim3 grid, cudaStream_t st
 // rounds of three: barrier stalls 5.4 per issued instruction) and one CTA's
 // loads overlap another's arithmetic.  Measured on GB300 (us): 8 transforms of
 // 2^20 124.9 -> 112.7 (2048-point rows), LDE 2^20 x 64 5589 -> 5130; one 2^20
-// (128 tiles) 23.1 -> 29.1, which is why the first form stays.
+// (128 tiles) 23.1 -> 29.1, which is why the first form stays.  PER_SM is per
+// shape, from 3, 4, 6 and 9 transforms of 512 x m (2.5, 3.4, 5.1 and 7.6 tiles
+// per SM), second form against first: m = 1280 0.84, 0.95, 1.06, 1.18 (four);
+// 2040 0.96, 0.96, 1.05, 1.04 (four); 1536 0.90, 1.03, 1.06, 1.15, 1360
+// and 2176 alike (three); 1088 1.15 .. 1.21, 1920, 2048, 2720 and 3264 1.03 and
+// up throughout (two).  m = 1024 stays at two (three transforms 27.4 us, with
+// the first form 28.8).
 template <int R1, int R2, int R3, int LANES, int NT, int NTM, int MINB, bool INV, int PER_SM = 2>
 static void gl_launch_pass3_by_tiles(const gl_pass_args &args, dim3 grid, cudaStream_t stream, bool pdl) {
   if ((uint64_t)grid.x * grid.y * grid.z > (uint64_t)PER_SM * (unsigned)gl_sm_count())
