@@ -210,6 +210,15 @@ const gl_kernel_entry *gl_find_kernel_cols(uint64_t m, bool inv) {
   return gl_find_kernel4(m, inv);
 }
 
+const gl_kernel_entry *gl_find_kernel_wide(uint64_t m, bool inv) {
+  size_t cnt = 0;
+  if (!use_two_lane_passes()) return nullptr;  // GOLDILOCKS_PASS_LANES=4
+  const gl_kernel_entry *e = inv ? gl_kernels_cols_inv(&cnt) : gl_kernels_cols_fwd(&cnt);
+  if (const gl_kernel_entry *k = find_in(e, cnt, m)) return k;
+  e = inv ? gl_kernels_wide_inv(&cnt) : gl_kernels_wide_fwd(&cnt);
+  return find_in(e, cnt, m);
+}
+
 const gl_kernel_entry *gl_find_kernel_gt(uint64_t m, bool inv) {
   size_t cnt = 0;
   const gl_kernel_entry *e = inv ? gl_kernels_gt17_inv(&cnt) : gl_kernels_gt17_fwd(&cnt);
@@ -244,9 +253,10 @@ extern "C" int gl_preload_kernels(void) {
   for (table_fn f : {gl_kernels_full_fwd, gl_kernels_full_inv, gl_kernels_full1_fwd, gl_kernels_full1_inv,
                      gl_kernels_gt17_fwd, gl_kernels_gt17_inv,
                      gl_kernels_pass_fwd, gl_kernels_pass_inv,
-                     gl_kernels_small_fwd, gl_kernels_small_inv, gl_kernels_mixed35_fwd, gl_kernels_mixed35_inv, gl_kernels_mixed17_fwd,
-                     gl_kernels_mixed17_inv, gl_kernels_pass2_fwd, gl_kernels_pass2_inv, gl_kernels_cols_fwd,
-                     gl_kernels_cols_inv}) {
+                     gl_kernels_small_fwd, gl_kernels_small_inv, gl_kernels_mixed35_fwd,
+                     gl_kernels_mixed35_inv, gl_kernels_mixed17_fwd, gl_kernels_mixed17_inv,
+                     gl_kernels_pass2_fwd, gl_kernels_pass2_inv, gl_kernels_cols_fwd, gl_kernels_cols_inv,
+                     gl_kernels_wide_fwd, gl_kernels_wide_inv}) {
     size_t n = 0;
     const gl_kernel_entry *e = f(&n);
     for (size_t i = 0; i < n; i++)
@@ -506,6 +516,10 @@ bool gl_choice_apply(gl_plan *pl, const gl_choice &c) {
         pl->k[c.kind - 1][d] = g;
         pl->k4[c.kind - 1][d] = g;
       }
+    }
+    for (int s = 0; c.kind >= 2 && s < c.kind; s++) {
+      const gl_kernel_entry *h = gl_find_kernel_wide(f[s], d == 1);
+      pl->kw[s][d] = h ? h : pl->k[s][d];
     }
   }
   return true;
@@ -988,6 +1002,29 @@ bool gl_first_pass_pdl(cudaStream_t stream, uint64_t tiles) {
   return cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }
 
+// The kernel of stage s of a two-pass plan for a launch of `items` contiguous
+// transforms with `lanes` lanes each: that of the schedule, or one of more lanes
+// where the launch has many tiles (and an item's last tile is nearly full).  Measured on GB300 (us, the schedule's
+// kernel -> this one):
+//   four lanes in 512 threads for two in 256 at 1024 and 2048 points, from more
+//   than two four-lane tiles per SM on: 2^22 67.2 -> 66.7, four of them 259 ->
+//   231, 2^23 142 -> 134 (a launch of fewer tiles keeps the two lanes);
+//   16 or 32 lanes (128- and 256-byte row pieces, 256 threads) for four in 32 or
+//   64 threads at up to 256 points: columns from one such tile per SM on, 256 x
+//   2^13 25.2 -> 20.9, 128 x 2^14 25.3 -> 21.5, 64 x 2^15 29.9 -> 25.4 (one 2^13,
+//   two wide tiles in all: 6.9 -> 8.3); rows from six on, 512 x 2^13 37.0 -> 36.5
+//   (16 x 2^16, 1.7 tiles per SM: 17.3 -> 20.2; 32 of them, 3.4: 25.3 -> 26.3).
+const gl_kernel_entry *gl_contiguous_pass(const gl_plan *pl, int s, int d, uint64_t lanes, uint64_t items) {
+  const gl_kernel_entry *k = pl->k[s][d], *k4 = pl->k4[s][d], *kw = pl->kw[s][d];
+  const uint64_t sms = (uint64_t)gl_sm_count();
+  if (k->lanes == 2 && k4->lanes == 4 && lanes / 4 * items > 2 * sms) return k4;
+  const uint64_t wide = gl_tiles(lanes, kw);
+  if (k->m <= 256 && kw->lanes > k->lanes && wide * items >= (s == 0 ? 1 : 6) * sms &&
+      wide * kw->lanes <= lanes + lanes / 8)
+    return kw;
+  return k;
+}
+
 // Queue the transform of a strided batch on `stream`.  Element j of column c
 // of batch item b is at base[b*bs + j*C + c] (C = 1, bs = n: contiguous
 // transforms; C = cols, B = 1: the columns of a row-major matrix).  `src` and
@@ -1087,8 +1124,14 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
     //   C  per (k1, k2): n3-point over j3, stored at k         scratch -> dst
     // (a column pass writes exactly the positions it reads, so B is in place).
     const uint64_t n1 = pl->n1, n2 = pl->n2, n3 = pl->n3, n23 = n2 * n3;
-    const auto &ks = C > 1 ? pl->k4 : pl->k;  // interleaved columns: four-lane kernels
-    const gl_kernel_entry *ka = ks[0][d], *kb = ks[1][d], *kcr = ks[2][d];
+    // Interleaved columns: four lanes or more in every pass.  Contiguous
+    // transforms (2^24 words and more): eight lanes or more for the column
+    // passes, since the 32-byte pieces of a four-lane tile lie up to a MB apart
+    // (us, 2^28 5788 -> 4997, 255 x 2^17 726 -> 667, 2^25 586 -> 582), and four
+    // for the rows, eight where they go to host memory (2^25 rows: two lanes
+    // 641, four 585, eight 590).
+    const gl_kernel_entry *ka = (C > 1 ? pl->k4 : pl->kw)[0][d], *kb = (C > 1 ? pl->k4 : pl->kw)[1][d];
+    const gl_kernel_entry *kcr = (lo->host && C == 1 ? pl->kw : pl->k4)[2][d];
     for (uint64_t b = 0; b < B; b++) {
       const uint64_t *in = src + b * bs;
       uint64_t *out = dst + b * bs;
@@ -1156,8 +1199,9 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
   }
   // Four-step: n = n1*n2, j = n2*j1 + j2, k = k1 + n1*k2.
   const uint64_t n1 = pl->n1, n2 = pl->n2;
-  const auto &ks = C > 1 ? pl->k4 : pl->k;  // interleaved columns: four-lane kernels
-  const gl_kernel_entry *kc = ks[0][d], *kr = ks[1][d];
+  const bool wide = C == 1 && lo->host;
+  const gl_kernel_entry *kc = C > 1 ? pl->k4[0][d] : wide ? pl->kw[0][d] : gl_contiguous_pass(pl, 0, d, n2, B);
+  const gl_kernel_entry *kr = C > 1 ? pl->k4[1][d] : wide ? pl->kw[1][d] : gl_contiguous_pass(pl, 1, d, n1, B);
   for (uint64_t off = 0; off < B; off += kMaxGridYZ) {
     const uint64_t cb = std::min(kMaxGridYZ, B - off);
     // COL: lanes are (j2, c) pairs, contiguous; n1-point transforms down them.
@@ -1235,7 +1279,7 @@ int gl_enqueue_pass_range(gl_plan *pl, int stage, const uint64_t *src, uint64_t 
   a.lanes = (uint32_t)(hi - lo);
   if (stage == 0) {
     if (hi > n2) return GL_ERR_INVALID;
-    const gl_kernel_entry *kc = pl->k[0][d];
+    const gl_kernel_entry *kc = gl_contiguous_pass(pl, 0, d, hi - lo, 1);
     a.in = src + lo; a.out = dst + lo;
     a.in_ls = a.out_ls = 1; a.in_is = a.out_is = (int64_t)n2;
     a.flags = GL_PF_PASS_TWIDDLE | GL_PF_LOAD_LANE_FAST | GL_PF_STORE_LANE_FAST;
@@ -1251,7 +1295,7 @@ int gl_enqueue_pass_range(gl_plan *pl, int stage, const uint64_t *src, uint64_t 
     gl_launch(kc, 1, a, dim3((unsigned)gl_tiles(hi - lo, kc)), n1 * (hi - lo), stream);
   } else {
     if (hi > n1) return GL_ERR_INVALID;
-    const gl_kernel_entry *kr = pl->k[1][d];
+    const gl_kernel_entry *kr = gl_contiguous_pass(pl, 1, d, hi - lo, 1);
     a.in = src + lo * n2; a.out = dst + lo;
     a.in_ls = (int64_t)n2; a.in_is = 1; a.out_ls = 1; a.out_is = (int64_t)n1;
     a.flags = GL_PF_STORE_LANE_FAST;
@@ -1349,8 +1393,18 @@ void *gl_host_device_view(const void *p, uint64_t bytes) {
   return a0.devicePointer;
 }
 
-// Host-memory calls from this many words on move in column blocks.
-static const uint64_t kHostBlocksMinWords = 1ull << 21;
+// Host-memory calls from this many words on take the passes of eight lanes or
+// more: pieces of 32 bytes cross the host link at 160 (in) and 129 GB/s (out),
+// pieces of 64 bytes at 171 and 157, copies at 192 and 179, but a short call
+// waits for the longer tiles.  Measured on GB300 (us, four lanes -> wide):
+// 2^16 points 28.6 -> 29.5, 2^18 49.0 -> 47.9, 2^19 78 -> 74, 2^20 136 -> 127,
+// 2 x 2^22 (two lanes) 2490 -> 772, 16 x 2^16 133 -> 113.
+static const uint64_t kHostWideMinWords = 1ull << 18;
+
+// Host-memory calls of one transform from this many words on move in column
+// blocks.  (us, in place -> in blocks: 2^21 points 237 -> 307, 17 x 2^17 257 ->
+// 271, 3 x 2^20 348 -> 344, 15 x 2^18 426 -> 408, 2^23 857 -> 771.)
+static const uint64_t kHostBlocksMinWords = 3ull << 20;
 
 static int execute(gl_plan *pl, uint64_t *data, uint64_t len, int dir, int mem, void *ws,
                    uint64_t ws_bytes, cudaStream_t stream) {
@@ -1398,7 +1452,9 @@ static int execute(gl_plan *pl, uint64_t *data, uint64_t len, int dir, int mem, 
       cudaError_t e = gl_malloc_async((void **)&scratch, need, stream);
       if (e != cudaSuccess) return gl_cuda_status(e);
     }
-    st = run_device(pl, hv, count, inv, scratch, stream);
+    gl_load_opts over;
+    over.host = len >= kHostWideMinWords;
+    st = gl_enqueue_transform(pl, hv, hv, 1, count, pl->size, inv, scratch, stream, &over);
     if (scratch) cudaFreeAsync(scratch, stream);
     cudaError_t e = cudaStreamSynchronize(stream);
     return st != GL_OK ? st : gl_cuda_status(e);

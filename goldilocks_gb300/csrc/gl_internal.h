@@ -115,6 +115,9 @@ const gl_kernel_entry *gl_find_kernel(uint64_t m, bool full, bool inv);
 const gl_kernel_entry *gl_find_kernel4(uint64_t m, bool inv);
 // The pass kernel for m over interleaved columns (C > 1).
 const gl_kernel_entry *gl_find_kernel_cols(uint64_t m, bool inv);
+const gl_kernel_entry *gl_find_kernel_wide(uint64_t m, bool inv);  // nullptr: none compiled
+const gl_kernel_entry *gl_kernels_wide_fwd(size_t *count);
+const gl_kernel_entry *gl_kernels_wide_inv(size_t *count);
 const gl_kernel_entry *gl_kernels_cols_fwd(size_t *count);
 const gl_kernel_entry *gl_kernels_cols_inv(size_t *count);
 
@@ -160,6 +163,10 @@ struct gl_plan {
   // CTA (a two-lane CTA would read and write 16-byte row pieces), 8-32 lanes
   // for passes up to 512 points.
   const gl_kernel_entry *k4[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
+  // The same stages (C = 1) in kernels of eight lanes or more where one is
+  // compiled, elsewhere k: contiguous launches of many tiles, three-pass
+  // columns, and passes that read or write host memory (64-byte pieces).
+  const gl_kernel_entry *kw[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
   // kind 1: the one-transform-per-CTA kernel (nullptr below 512 points).
   const gl_kernel_entry *k1[2] = {nullptr, nullptr};
   std::string tree;
@@ -196,6 +203,7 @@ struct gl_load_opts {
   uint32_t in_limit = 0xffffffffu;   // rows >= in_limit read as zero
   const uint64_t *itw_lo = nullptr;  // g^e, e < 4096
   const uint64_t *itw_hi = nullptr;  // g^(4096 e)
+  bool host = false;                 // src and dst are host memory
 };
 
 // Optional store-side pointwise product on the last pass of a forward
@@ -244,6 +252,8 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
                          uint64_t bs, bool inv, uint64_t *scratch, cudaStream_t stream,
                          const gl_load_opts *lo = nullptr, const gl_store_mul *om = nullptr,
                          uint64_t out_row = 0);
+
+const gl_kernel_entry *gl_contiguous_pass(const gl_plan *pl, int s, int d, uint64_t lanes, uint64_t items);
 
 // Queue a batch on the persistent kernel without waiting; the kernel's error
 // word (0 = success) is copied to *err_out afterwards.  (gl_batch.cu)

@@ -25,6 +25,18 @@ static const gl_kernel_entry k_col_entries[] = {
     GL_ENTRY3C(8, 8, 1, 32, 256, 4, true),
 };
 
+// 1024 and 2048 points in eight lanes: with the entries above, the passes that
+// read or write host memory (64-byte pieces) and three-pass columns.
+static const gl_kernel_entry k_wide_entries[] = {
+    GL_ENTRY3M(16, 8, 8, 8, 512, 2, true),
+    GL_ENTRY3M(16, 16, 8, 8, 1024, 1, true),
+};
+
+const gl_kernel_entry *gl_kernels_wide_inv(size_t *count) {
+  *count = sizeof(k_wide_entries) / sizeof(k_wide_entries[0]);
+  return k_wide_entries;
+}
+
 const gl_kernel_entry *gl_kernels_cols_inv(size_t *count) {
   *count = sizeof(k_col_entries) / sizeof(k_col_entries[0]);
   return k_col_entries;
