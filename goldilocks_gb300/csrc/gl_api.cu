@@ -1025,6 +1025,17 @@ const gl_kernel_entry *gl_contiguous_pass(const gl_plan *pl, int s, int d, uint6
   return k;
 }
 
+// The kernel of the second pass over C interleaved columns with `rows` rows in
+// the launch.  At 1024 and 2048 points eight lanes (64-byte row pieces, one
+// 1024-thread CTA per SM at 2048) for four where whole tiles of them give every
+// SM 12: 2^20 x 64 columns 847 -> 832 us, LDE of 2^20 x 32 to twice the length
+// 1397 -> 1371, 2^20 x 32 columns 424 -> 423; 2^20 x 8 (3.4 tiles) 105 -> 113.
+static const gl_kernel_entry *gl_column_rows(const gl_plan *pl, int d, uint64_t C, uint64_t rows) {
+  const gl_kernel_entry *k = pl->k4[1][d], *kw = pl->kw[1][d];
+  const bool wider = k->lanes == 4 && kw->lanes == 8 && k->m >= 1024;
+  return wider && C % 8 == 0 && C / 8 * rows >= 12ull * (unsigned)gl_sm_count() ? kw : k;
+}
+
 // Queue the transform of a strided batch on `stream`.  Element j of column c
 // of batch item b is at base[b*bs + j*C + c] (C = 1, bs = n: contiguous
 // transforms; C = cols, B = 1: the columns of a row-major matrix).  `src` and
@@ -1201,7 +1212,7 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
   const uint64_t n1 = pl->n1, n2 = pl->n2;
   const bool wide = C == 1 && lo->host;
   const gl_kernel_entry *kc = C > 1 ? pl->k4[0][d] : wide ? pl->kw[0][d] : gl_contiguous_pass(pl, 0, d, n2, B);
-  const gl_kernel_entry *kr = C > 1 ? pl->k4[1][d] : wide ? pl->kw[1][d] : gl_contiguous_pass(pl, 1, d, n1, B);
+  const gl_kernel_entry *kr = C > 1 ? gl_column_rows(pl, d, C, n1 * B) : wide ? pl->kw[1][d] : gl_contiguous_pass(pl, 1, d, n1, B);
   for (uint64_t off = 0; off < B; off += kMaxGridYZ) {
     const uint64_t cb = std::min(kMaxGridYZ, B - off);
     // COL: lanes are (j2, c) pairs, contiguous; n1-point transforms down them.

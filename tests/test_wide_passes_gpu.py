@@ -65,3 +65,19 @@ def test_three_passes(oracle, n):
     a = torch.from_numpy(x.view(np.int64).copy()).pin_memory().numpy().view(np.uint64)
     plan.ntt(a)
     assert np.array_equal(a, got)
+
+
+@pytest.mark.parametrize("n,cols", [(1 << 19, 24), (1 << 19, 32), (1 << 19, 30), (1 << 20, 32)])
+@pytest.mark.parametrize("inv", [False, True])
+def test_column_rows(n, cols, inv):
+    import torch
+    import goldilocks_gb300 as gl
+    from goldilocks_gb300 import _lib
+    x = rand_field(n * cols, seed=cols + inv).reshape(n, cols)
+    t = torch.from_numpy(x.view(np.int64).copy()).cuda()
+    assert _lib.load().gl_ntt_columns(t.data_ptr(), n, cols, _lib.GL_INVERSE if inv else _lib.GL_FORWARD,
+                                      _lib.GL_MEM_DEVICE, torch.cuda.current_stream().cuda_stream) == _lib.GL_OK
+    got = t.cpu().numpy().view(np.uint64)
+    plan = gl.strategy(n)
+    for c in range(0, cols, 3):
+        assert np.array_equal(got[:, c], device(plan, np.ascontiguousarray(x[:, c]), inv)), c
