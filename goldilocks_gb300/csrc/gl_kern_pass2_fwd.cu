@@ -1,9 +1,7 @@
-// Four-step column/row pass kernels for pass sizes up to 2048: two lanes per
-// 256-thread CTA and four CTAs per SM, so that one CTA's loads overlap the
-// others' arithmetic (forward).  Measured on GB300 against the
-// four-lane 1024-thread kernels: 2048-point passes 12-17 % faster, 1024-point
-// column passes 8 %; at 4096 points the same split (512 threads, two CTAs)
-// was 2-8 % slower, so those keep four lanes.
+// Four-step column/row pass kernels of 1024 and 2048 points with two lanes per
+// 256-thread CTA and four CTAs per SM (forward): the schedules nearest sqrt(n),
+// for launches of up to two four-lane tiles per SM.  More tiles take the
+// four-lane kernels in 512 threads (measured at gl_contiguous_pass).
 #include "gl_kernels_impl.cuh"
 
 static const gl_kernel_entry k_entries[] = {
