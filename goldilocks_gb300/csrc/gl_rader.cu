@@ -18,11 +18,13 @@
 //   scatter    Y[j2][k1] = (x0 + A[p]) * omega_n^(j2 k1), k1 = g^-p; Y[j2][0] = X0 * 1
 //   transform  Y (m rows, q*C columns) with the plan of m -> X
 // Rows are contiguous across lanes (l = j2*C + c), so gather, pointwise and
-// the column transforms read and write whole rows.
+// the column transforms read and write whole rows.  For q = 257 all steps but the
+// last are one kernel (gl_rader257.cuh).
 #include <algorithm>
 #include <vector>
 
 #include "gl_internal.h"
+#include "gl_rader257.cuh"
 
 namespace {
 
@@ -86,7 +88,7 @@ __global__ void gl_rader_pointwise_kernel(uint64_t *A, const uint64_t *x0, uint6
     const uint64_t p = i / L;
     const uint64_t a = A[i];
     if (p == 0) X0[i] = gl_add(x0[i], a);
-    A[i] = gl_mul(a, __ldg(bhat + p));
+    A[i] = gl_mont_mul(a, __ldg(bhat + p));
   }
 }
 
@@ -111,7 +113,7 @@ __global__ void gl_rader_scatter_kernel(const uint64_t *conv, const uint64_t *x0
       v = gl_add(x0[l], conv[i - L]);
       k1 = gneg[r - 1];
     }
-    v = gl_mul(v, gl_tw2(tw_lo, tw_hi, j2 * k1));
+    v = gl_mont_mul(v, gl_tw2m(tw_lo, tw_hi, j2 * k1));
     Y[(j2 * q + k1) * C + c] = v;
   }
 }
@@ -138,9 +140,14 @@ __global__ void __launch_bounds__(256) gl_rader_scatter_tiled_kernel(
     const uint64_t l = l0 + i, k1 = k0 + threadIdx.x;
     if (k1 < q && l < L) {
       const uint64_t j2 = l / C, c = l - j2 * C;
-      Y[(j2 * q + k1) * C + c] = gl_mul(tile[threadIdx.x][i], gl_tw2(tw_lo, tw_hi, j2 * k1));
+      Y[(j2 * q + k1) * C + c] = gl_mont_mul(tile[threadIdx.x][i], gl_tw2m(tw_lo, tw_hi, j2 * k1));
     }
   }
+}
+
+__global__ void __launch_bounds__(GL_R257_NT, 1024 / GL_R257_NT) gl_rader257_kernel(const gl_rader257_args a) {
+  __shared__ uint64_t sm[GL_R257_SMEM];
+  gl_rader257_block(a, blockIdx.x, sm);
 }
 
 int gl_rader_tables(gl_plan *pl, gl_dev_tables &t) {
@@ -163,16 +170,16 @@ int gl_rader_tables(gl_plan *pl, gl_dev_tables &t) {
     const uint64_t w = root(n, d == 1);
     std::vector<uint64_t> lo(GL_TW_SPLIT), hi(hi_count);
     uint64_t x = d == 1 ? gl_inv(q) : 1;
-    for (uint64_t e = 0; e < GL_TW_SPLIT; e++) { lo[e] = x; x = gl_mul(x, w); }
+    for (uint64_t e = 0; e < GL_TW_SPLIT; e++) { lo[e] = gl_to_mont(x); x = gl_mul(x, w); }
     const uint64_t w4096 = gl_pow(w, GL_TW_SPLIT);
     x = 1;
-    for (uint64_t e = 0; e < hi_count; e++) { hi[e] = x; x = gl_mul(x, w4096); }
+    for (uint64_t e = 0; e < hi_count; e++) { hi[e] = gl_to_mont(x); x = gl_mul(x, w4096); }
     st = upload(t, lo, &t.rader_tw_lo[d]);
     if (st == GL_OK) st = upload(t, hi, &t.rader_tw_hi[d]);
-    // b_s = omega_q^(g^-s), then its forward transform of length q - 1.
+    // b_s = omega_q^(g^-s) in Montgomery form (as all tables), then its forward transform of length q - 1.
     std::vector<uint64_t> bv(r);
     const uint64_t wq = root(q, d == 1);
-    for (uint64_t s = 0; s < r; s++) bv[s] = gl_pow(wq, gn[s]);
+    for (uint64_t s = 0; s < r; s++) bv[s] = gl_to_mont(gl_pow(wq, gn[s]));
     if (st == GL_OK) st = upload(t, bv, &t.rader_bhat[d]);
     if (st != GL_OK) break;
     // Transformed on the table stream, after its upload there; the caller
@@ -204,9 +211,28 @@ int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C
   uint64_t *A = scratch, *x0 = A + r * L, *X0 = x0 + L;
   uint64_t *Y = X0 + L;
   uint64_t *sub = Y + (m > 1 ? n * C : 0);
+  // The fused kernel takes the one-pass tables of 256 points (a tuned plan of
+  // 256 in two passes has others) and up to 2^31 - 1 tiles.
+  gl_dev_tables *tq = nullptr;
+  const bool fused = q == 257 && pl->pq->kind == 1 && (L + GL_R257_LANES - 1) / GL_R257_LANES <= 0x7fffffffull;
+  if (fused && (st = gl_plan_tables(pl->pq, &tq)) != GL_OK) return st;
   for (uint64_t b = 0; b < B; b++) {
     const uint64_t *in = src + b * bs;
     uint64_t *out = dst + b * bs;
+    if (fused) {
+      gl_rader257_args a{};
+      a.src = in; a.dst = m > 1 ? Y : out; a.L = L; a.C = C;
+      a.gpow = t->rader_gpow; a.gneg = t->rader_gneg;
+      a.tw_f = tq->blk[0][0]; a.tw_i = tq->blk_scaled_inv; a.bhat = t->rader_bhat[d];
+      a.tw_lo = t->rader_tw_lo[d]; a.tw_hi = t->rader_tw_hi[d];
+      const uint64_t tiles = (L + GL_R257_LANES - 1) / GL_R257_LANES;
+      if ((st = launch(gl_rader257_kernel, dim3((unsigned)tiles), GL_R257_NT, stream,
+                       b > 0 || gl_first_pass_pdl(stream, tiles), a)) != GL_OK)
+        return st;
+      if (m > 1 && (st = gl_enqueue_transform(pl->pm, Y, out, q * C, 1, n * C, inv, sub, stream)) != GL_OK)
+        return st;
+      continue;
+    }
     if ((st = launch(gl_rader_gather_kernel, grid_for(q * L), 256, stream, b > 0 || gl_first_pass_pdl(stream, 0), in,
                      A, x0, t->rader_gpow, L, q)) != GL_OK)
       return st;
@@ -230,6 +256,7 @@ int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C
 }
 
 void gl_rader_kernels(std::vector<const void *> &out) {
+  out.push_back((const void *)gl_rader257_kernel);
   out.push_back((const void *)gl_rader_gather_kernel);
   out.push_back((const void *)gl_rader_pointwise_kernel);
   out.push_back((const void *)gl_rader_scatter_kernel);
