@@ -145,9 +145,21 @@ __global__ void __launch_bounds__(256) gl_rader_scatter_tiled_kernel(
   }
 }
 
-__global__ void __launch_bounds__(GL_R257_NT, 1024 / GL_R257_NT) gl_rader257_kernel(const gl_rader257_args a) {
-  __shared__ uint64_t sm[GL_R257_SMEM];
-  gl_rader257_block(a, blockIdx.x, sm);
+template <int LN>
+__global__ void __launch_bounds__(LN * 16, 64 / LN) gl_rader257_kernel(const gl_rader257_args a) {
+  __shared__ uint64_t sm[LN * 272];
+  gl_rader257_block<LN>(a, blockIdx.x, sm);
+}
+
+// Eight lanes while they give every SM at most one tile, else sixteen (128-byte
+// rows).  us, 16 -> 8 lanes: 257 x 1024 23.8 -> 21.8, 257 12.6 -> 11.4, 257 x 64 26.9 ->
+// 28.2; 257 x 3840 48.9 -> 50.0, 257 x 65536 361 -> 374 (four lanes 378).
+static int rader257(const gl_rader257_args &a, cudaStream_t stream, bool early) {
+  const int lanes = a.L <= 8ull * (unsigned)gl_sm_count() ? 8 : 16;
+  const uint64_t tiles = (a.L + lanes - 1) / lanes;
+  const bool pdl = early || gl_first_pass_pdl(stream, tiles);
+  return launch(lanes == 8 ? gl_rader257_kernel<8> : gl_rader257_kernel<16>, dim3((unsigned)tiles), lanes * 16, stream,
+                pdl, a);
 }
 
 int gl_rader_tables(gl_plan *pl, gl_dev_tables &t) {
@@ -214,7 +226,7 @@ int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C
   // The fused kernel takes the one-pass tables of 256 points (a tuned plan of
   // 256 in two passes has others) and up to 2^31 - 1 tiles.
   gl_dev_tables *tq = nullptr;
-  const bool fused = q == 257 && pl->pq->kind == 1 && (L + GL_R257_LANES - 1) / GL_R257_LANES <= 0x7fffffffull;
+  const bool fused = q == 257 && pl->pq->kind == 1 && L / 16 < 0x7fffffffull;
   if (fused && (st = gl_plan_tables(pl->pq, &tq)) != GL_OK) return st;
   for (uint64_t b = 0; b < B; b++) {
     const uint64_t *in = src + b * bs;
@@ -225,10 +237,7 @@ int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C
       a.gpow = t->rader_gpow; a.gneg = t->rader_gneg;
       a.tw_f = tq->blk[0][0]; a.tw_i = tq->blk_scaled_inv; a.bhat = t->rader_bhat[d];
       a.tw_lo = t->rader_tw_lo[d]; a.tw_hi = t->rader_tw_hi[d];
-      const uint64_t tiles = (L + GL_R257_LANES - 1) / GL_R257_LANES;
-      if ((st = launch(gl_rader257_kernel, dim3((unsigned)tiles), GL_R257_NT, stream,
-                       b > 0 || gl_first_pass_pdl(stream, tiles), a)) != GL_OK)
-        return st;
+      if ((st = rader257(a, stream, b > 0)) != GL_OK) return st;
       if (m > 1 && (st = gl_enqueue_transform(pl->pm, Y, out, q * C, 1, n * C, inv, sub, stream)) != GL_OK)
         return st;
       continue;
@@ -256,7 +265,8 @@ int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C
 }
 
 void gl_rader_kernels(std::vector<const void *> &out) {
-  out.push_back((const void *)gl_rader257_kernel);
+  out.push_back((const void *)gl_rader257_kernel<8>);
+  out.push_back((const void *)gl_rader257_kernel<16>);
   out.push_back((const void *)gl_rader_gather_kernel);
   out.push_back((const void *)gl_rader_pointwise_kernel);
   out.push_back((const void *)gl_rader_scatter_kernel);

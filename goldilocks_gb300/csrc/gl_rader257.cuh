@@ -1,7 +1,7 @@
 // The whole Rader step over the factor 257 in one kernel (m = n / 257 lanes of
 // C columns, L = m*C lanes): gather, 256-point transform, product with the
-// transformed Rader kernel, inverse transform, x[0] and twiddle, for 16 adjacent
-// lanes per 256-thread CTA.
+// transformed Rader kernel, inverse transform, x[0] and twiddle, for LN adjacent
+// lanes per CTA of 16*LN threads and 272*LN words of shared memory.
 //
 // Both transforms are 16 x 16, a thread's 16-point group in registers.  The first
 // leaves frequency k1 + 16 t at t of the thread of group k1, which is the input
@@ -11,7 +11,7 @@
 // step took five kernels and about nine passes over memory.  Bound by the
 // integer pipes and, for few tiles, by the four codelets in a row of each thread.
 // Whole transforms on GB300 (us, before -> now): 257 x 4096 45.9 -> 38.0, 257 x
-// 65536 545 -> 361, 257 x 256 over 64 columns 111 -> 66, one 257 15.1 -> 12.6.
+// 65536 545 -> 361, 257 x 256 over 64 columns 111 -> 66, one 257 15.1 -> 11.3.
 #pragma once
 #include "gl_pass.cuh"
 
@@ -27,12 +27,8 @@ struct gl_rader257_args {
   const uint64_t *tw_lo, *tw_hi;  // omega_n^e (Montgomery form, perhaps scaled)
 };
 
-constexpr int GL_R257_LANES = 16, GL_R257_NT = 16 * GL_R257_LANES;
-constexpr int GL_R257_SMEM = GL_R257_LANES * 272;  // words
-constexpr int GL_R257_WORDS = GL_R257_LANES * 257;
-
+template <int LN>
 __device__ __forceinline__ void gl_rader257_block(const gl_rader257_args &a, uint64_t bx, uint64_t *sm) {
-  constexpr int LN = GL_R257_LANES;
   const uint32_t c = threadIdx.x % LN, g = threadIdx.x / LN;
   const uint64_t l = bx * LN + c;
   const bool live = l < a.L;
@@ -82,7 +78,7 @@ __device__ __forceinline__ void gl_rader257_block(const gl_rader257_args &a, uin
   }
   if (!block) return;
   __syncthreads();
-  const uint64_t first = bx * GL_R257_WORDS, end = a.L * 257;
-  for (int i = threadIdx.x; i < GL_R257_WORDS; i += GL_R257_NT)
+  const uint64_t first = bx * (LN * 257), end = a.L * 257;
+  for (int i = threadIdx.x; i < LN * 257; i += LN * 16)
     if (first + i < end) a.dst[first + i] = sm[i];
 }

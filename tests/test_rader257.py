@@ -14,19 +14,24 @@ from test_kernel_emulation import root, table
 HARNESS = r"""
 #include "kernel_emu.cpp"
 #include "gl_rader257.cuh"
-extern "C" void emu_rader257(const uint64_t *src, uint64_t *dst, uint64_t L, uint64_t C, const uint32_t *gp,
+template <int LN>
+static void run(const gl_rader257_args &a) {
+  for (uint64_t x = 0; x < (a.L + LN - 1) / LN; x++) {
+    memset(sm, 0xA5, sizeof(sm));
+    std::barrier<> bar(LN * 16);
+    g_bar = &bar;
+    std::vector<std::thread> th;
+    for (int t = 0; t < LN * 16; t++)
+      th.emplace_back([&a, t, x] { threadIdx.x = t; gl_rader257_block<LN>(a, x, sm); });
+    for (auto &t : th) t.join();
+  }
+}
+extern "C" void emu_rader257(int lanes, const uint64_t *src, uint64_t *dst, uint64_t L, uint64_t C, const uint32_t *gp,
                              const uint32_t *gn, const uint64_t *tf, const uint64_t *ti, const uint64_t *bhat,
                              const uint64_t *lo, const uint64_t *hi) {
   const gl_rader257_args a{src, dst, L, C, gp, gn, tf, ti, bhat, lo, hi};
-  for (uint64_t x = 0; x < (L + GL_R257_LANES - 1) / GL_R257_LANES; x++) {
-    memset(sm, 0xA5, sizeof(sm));
-    std::barrier<> bar(GL_R257_NT);
-    g_bar = &bar;
-    std::vector<std::thread> th;
-    for (int t = 0; t < GL_R257_NT; t++)
-      th.emplace_back([&a, t, x] { threadIdx.x = t; gl_rader257_block(a, x, sm); });
-    for (auto &t : th) t.join();
-  }
+  if (lanes == 8) run<8>(a);
+  else run<16>(a);
 }
 """
 
@@ -39,13 +44,14 @@ def emu(tmp_path_factory):
                     "-I" + os.path.join(ROOT, "goldilocks_gb300", "csrc"), "-I" + os.path.join(ROOT, "tests"),
                     str(d / "r.cpp"), "-o", str(d / "r.so")], check=True)
     lib = ctypes.CDLL(str(d / "r.so"))
-    lib.emu_rader257.argtypes = [ctypes.c_void_p] * 2 + [ctypes.c_uint64] * 2 + [ctypes.c_void_p] * 7
+    lib.emu_rader257.argtypes = [ctypes.c_int] + [ctypes.c_void_p] * 2 + [ctypes.c_uint64] * 2 + [ctypes.c_void_p] * 7
     return lib
 
 
 @pytest.mark.parametrize("m,C", [(1, 1), (16, 1), (17, 1), (48, 1), (1, 3), (8, 3), (2, 16), (1, 20)])
 @pytest.mark.parametrize("inv", [False, True])
-def test_fused_step(emu, oracle, m, C, inv):
+@pytest.mark.parametrize("lanes", [8, 16])
+def test_fused_step(emu, oracle, m, C, inv, lanes):
     n, L = 257 * m, m * C
     w = root(n, inv)
     gp = np.array([pow(3, p, 257) for p in range(256)], dtype=np.uint32)
@@ -60,7 +66,8 @@ def test_fused_step(emu, oracle, m, C, inv):
     x = rand_field(257 * L, seed=L + inv)
     x[:2] = 2**64 - 1
     out = np.full_like(x, 0x5555)
-    emu.emu_rader257(x.ctypes.data, out.ctypes.data, L, C, *(a.ctypes.data for a in (gp, gn, tf, ti, bhat, lo, hi)))
+    tables = (gp, gn, tf, ti, bhat, lo, hi)
+    emu.emu_rader257(lanes, x.ctypes.data, out.ctypes.data, L, C, *(a.ctypes.data for a in tables))
     rows = x.reshape(257, L)
     for l in range(0, L, 5 if L > 8 else 1):
         y = (oracle.intt if inv else oracle.ntt)(rows[:, l] % np.uint64(P))
