@@ -1208,6 +1208,15 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
     }
     return gl_cuda_status(cudaGetLastError());
   }
+  // About one column tile per SM: launched beside a row pass that leaves SMs
+  // free, the tiles crowd on those.  us, early -> not: 393 216 points (192 tiles)
+  // 17.6 -> 15.1, 2^18 (128) 13.4 -> 12.1, 2^19 (256) 15.6 -> 15.2, 327 680 (160)
+  // 14.4 -> 15.0; outside, 2^17 (64) 9.0 -> 11.0, 655 360 (320) 18.0 -> 19.1, and
+  // tiles of 32 or 64 threads do not crowd: 2^15 (128 of 64 points) 7.0 -> 10.7.
+  auto uneven = [&](uint64_t tiles) {
+    const uint64_t sms = (uint64_t)gl_sm_count();
+    return C == 1 && pl->n1 >= 512 && 6 * tiles >= 5 * sms && tiles <= 2 * sms;
+  };
   // Four-step: n = n1*n2, j = n2*j1 + j2, k = k1 + n1*k2.
   const uint64_t n1 = pl->n1, n2 = pl->n2;
   const bool wide = C == 1 && lo->host;
@@ -1238,7 +1247,7 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
     const uint64_t lanes1 = n2 * C;
     if (gl_tiles(lanes1, kc) > 0x7fffffffull) return GL_ERR_INVALID;
     gl_launch(kc, 1, a, dim3((unsigned)gl_tiles(lanes1, kc), (unsigned)cb),
-              cb * n * C, stream, off > 0 || pdl(gl_tiles(lanes1, kc) * cb));
+              cb * n * C, stream, off > 0 || (pdl(gl_tiles(lanes1, kc) * cb) && !uneven(gl_tiles(lanes1, kc) * cb)));
     // ROW: n2-point transforms along j2 for every (k1, c); transposed store.
     gl_pass_args b = base_args();
     b.in_limit = 0xffffffffu;  // zero padding applies to the first pass only
