@@ -7,7 +7,8 @@ Each entry is a contiguous CUDA int64/uint64 tensor transformed in place (its
 length must divide p - 1).  Modes: PERSISTENT (one launch, device work queue),
 BUCKETS (per-size launches replayed from a CUDA graph), PER_CALL (one call per
 polynomial), AUTO (the mode `autotune` measured fastest for this batch shape,
-else BUCKETS).  `run_packed` takes the polynomials as (offset, length,
+else BUCKETS).  Entries should not share memory: a batch in which some do runs
+one call after another (the order: gl_batch_execute in the header).  `run_packed` takes the polynomials as (offset, length,
 direction) arrays over one pool tensor.
 """
 import ctypes

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/goldilocks_gpu.h"
+#include "gl_batch_plan.h"
 #include "gl_internal.h"
 
 namespace {
@@ -536,6 +537,18 @@ int run_per_call(const gl_poly *polys, uint64_t count, cudaStream_t stream, bool
   return sync ? gl_cuda_status(cudaStreamSynchronize(stream)) : GL_OK;
 }
 
+// Polynomials that share memory, one after another: neither the branches of a
+// bucket graph nor the work items of the persistent kernel are ordered, so two
+// of them would race there.
+int run_in_order(const gl_poly *polys, uint64_t count, const std::vector<poly_plan> &pp, cudaStream_t stream) {
+  std::vector<bool> plain(count);
+  for (uint64_t i = 0; i < count; i++) plain[i] = pp[i].pl->kind >= 3;
+  std::vector<gl_poly> list;
+  list.reserve(count);
+  for (uint64_t i : gl_batch_order(polys, count, plain)) list.push_back(polys[i]);
+  return run_per_call(list.data(), count, stream);
+}
+
 // Autotuned choice per batch shape.
 std::mutex g_tune_mu;
 std::map<std::vector<std::pair<uint64_t, int>>, int> g_tuned;
@@ -574,6 +587,7 @@ extern "C" int gl_batch_execute(const gl_poly *polys, uint64_t count, int mode, 
     auto it = g_tuned.find(batch_shape(polys, count));
     mode = it != g_tuned.end() ? it->second : GL_BATCH_BUCKETS;  // the faster one untuned
   }
+  if (gl_batch_shares_memory(polys, count)) return run_in_order(polys, count, pp, stream);
   if (mode == GL_BATCH_PERSISTENT) return run_persistent(polys, count, pp, stream);
   return run_buckets(polys, count, pp, stream);
 }

@@ -235,7 +235,11 @@ enum { GL_BATCH_AUTO = 0, GL_BATCH_PERSISTENT = 1, GL_BATCH_BUCKETS = 2, GL_BATC
  * polynomial; GL_BATCH_AUTO: the mode gl_batch_autotune chose for this batch
  * shape, else buckets.  Sizes the persistent and bucket kernels are not
  * built for run per call.  Bounded waits: GL_ERR_TIMEOUT if a dependency did
- * not complete within 2 s. */
+ * not complete within 2 s.
+ * Polynomials should not share memory.  A batch in which some do runs one call
+ * after another: under GL_BATCH_PER_CALL in list order, else first the lengths
+ * of three passes or a Rader step in list order, then the others by (len, dir),
+ * equal ones in list order. */
 int gl_batch_execute(const gl_poly *polys, uint64_t count, int mode, void *stream);
 /* Time the three explicit modes (`reps` runs each; mean ms written to
  * ms_out[0..2] when non-null) and remember the fastest for this batch shape.
