@@ -352,8 +352,7 @@ struct bucket_graph {
   cudaGraphExec_t exec = nullptr;
   void *tables = nullptr;                  // pointer tables (device)
   size_t table_words = 0;
-  std::vector<std::pair<uint64_t, int>> sig;  // (len, dir) per item, bucket order
-  std::vector<const gl_plan *> plans;         // the plan of each item when captured
+  std::vector<const gl_plan *> plans;  // the plan of each item when captured
   ~bucket_graph() {
     if (exec) cudaGraphExecDestroy(exec);
     if (tables) cudaFree(tables);
@@ -361,7 +360,7 @@ struct bucket_graph {
 };
 
 std::mutex g_graph_mu;
-std::map<std::vector<std::pair<uint64_t, int>>, std::unique_ptr<bucket_graph>> g_graphs;
+std::map<gl_bucket_key, std::unique_ptr<bucket_graph>> g_graphs;
 
 // Streams a bucket graph is captured on: s[0] begins the capture, the others
 // fork from it and join it again.
@@ -433,8 +432,11 @@ int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_pla
   }
   std::vector<const gl_plan *> plans(nitems);
   for (size_t j = 0; j < nitems; j++) plans[j] = pp[order[j]].pl;
+  gl_bucket_key key{0, std::move(sig)};
+  if ((e = cudaGetDevice(&key.device)) != cudaSuccess) return gl_cuda_status(e);
+  const auto &items = key.sig;
   std::lock_guard<std::mutex> lk(g_graph_mu);
-  auto &slot = g_graphs[sig];
+  auto &slot = g_graphs[key];
   if (slot && slot->plans != plans) {
     // A schedule of one of the sizes changed (tuned or loaded) since the
     // capture: capture again with the current plans.
@@ -443,12 +445,11 @@ int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_pla
   }
   if (!slot) {
     auto g = std::make_unique<bucket_graph>();
-    g->sig = sig;
     g->plans = plans;
     g->table_words = flat.size();
     if ((e = cudaMalloc(&g->tables, flat.size() * sizeof(void *))) != cudaSuccess) {
       g->tables = nullptr;
-      g_graphs.erase(sig);
+      g_graphs.erase(key);
       return gl_cuda_status(e);
     }
     uint64_t **dt = (uint64_t **)g->tables;
@@ -463,10 +464,10 @@ int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_pla
     cudaGraph_t graph;
     std::vector<std::pair<size_t, size_t>> runs;  // items [first, end) of a bucket
     for (size_t j = 0, j1; j < nitems; j = j1) {
-      for (j1 = j; j1 < nitems && sig[j1] == sig[j];) j1++;
+      for (j1 = j; j1 < nitems && items[j1] == items[j];) j1++;
       runs.push_back({j, j1});
     }
-    auto work = [&](const std::pair<size_t, size_t> &r) { return sig[r.first].first * (r.second - r.first); };
+    auto work = [&](const std::pair<size_t, size_t> &r) { return items[r.first].first * (r.second - r.first); };
     std::stable_sort(runs.begin(), runs.end(), [&](const auto &x, const auto &y) { return work(x) > work(y); });
     uint64_t load[kBranches] = {};
     e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
@@ -512,7 +513,7 @@ int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_pla
     if (e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, graph, 0);
     if (e2 == cudaSuccess) cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
-      g_graphs.erase(sig);  // g frees its tables
+      g_graphs.erase(key);  // g frees its tables
       return gl_cuda_status(e);
     }
     slot = std::move(g);

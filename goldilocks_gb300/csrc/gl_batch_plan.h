@@ -40,3 +40,11 @@ inline std::vector<uint64_t> gl_batch_order(const gl_poly *polys, uint64_t count
   });
   return order;
 }
+
+// What a captured bucket graph is kept under: its kernel nodes, their tables
+// and the kernels chosen for its SMs belong to one device.
+struct gl_bucket_key {
+  int device;
+  std::vector<std::pair<uint64_t, int>> sig;  // (len, dir) per item, bucket order
+  bool operator<(const gl_bucket_key &o) const { return device != o.device ? device < o.device : sig < o.sig; }
+};
