@@ -462,14 +462,11 @@ int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_pla
     if ((e = br.create()) != cudaSuccess) return gl_cuda_status(e);
     cudaStream_t cap = br.s[0];
     cudaGraph_t graph;
-    std::vector<std::pair<size_t, size_t>> runs;  // items [first, end) of a bucket
-    for (size_t j = 0, j1; j < nitems; j = j1) {
-      for (j1 = j; j1 < nitems && items[j1] == items[j];) j1++;
-      runs.push_back({j, j1});
-    }
+    auto runs = gl_bucket_runs(items, 65535);  // grid.y
     auto work = [&](const std::pair<size_t, size_t> &r) { return items[r.first].first * (r.second - r.first); };
     std::stable_sort(runs.begin(), runs.end(), [&](const auto &x, const auto &y) { return work(x) > work(y); });
     uint64_t load[kBranches] = {};
+    cudaGetLastError();  // what an earlier call left is not a launch's below
     e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) e = br.fork();
     for (const auto &r : runs) {
@@ -506,6 +503,7 @@ int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_pla
         gl_launch(kr, 2, row, dim3((unsigned)gl_tiles(pl->n1, kr), (unsigned)(j1 - j)),
                   pl->size * (j1 - j), on, true);
       }
+      e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = br.join();
     cudaError_t e2 = cudaStreamEndCapture(cap, &graph);

@@ -48,3 +48,15 @@ struct gl_bucket_key {
   std::vector<std::pair<uint64_t, int>> sig;  // (len, dir) per item, bucket order
   bool operator<(const gl_bucket_key &o) const { return device != o.device ? device < o.device : sig < o.sig; }
 };
+
+// The launches of a bucket graph, as items [first, end): a bucket's items in one
+// launch, or in several of `most` (a launch has them on grid.y) items or fewer.
+inline std::vector<std::pair<size_t, size_t>> gl_bucket_runs(const std::vector<std::pair<uint64_t, int>> &sig,
+                                                             size_t most) {
+  std::vector<std::pair<size_t, size_t>> runs;
+  for (size_t j = 0, end; j < sig.size(); j = end) {
+    for (end = j + 1; end < sig.size() && end - j < most && sig[end] == sig[j];) end++;
+    runs.push_back({j, end});
+  }
+  return runs;
+}
