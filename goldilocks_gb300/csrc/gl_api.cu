@@ -245,7 +245,8 @@ __global__ void gl_coset_pad_kernel(const uint64_t *coef, uint64_t *dst, uint64_
 // on its first launch, and that load waits for the work already running on
 // the device: the first request of a new shape would wait for a long request
 // on another stream.  Querying a kernel's attributes loads it, so this loads
-// every kernel the library can launch.
+// every kernel the library can launch but the autotuner's (gl_tune.cu) and the
+// field check's (gl_debug.cu) own.
 extern "C" int gl_preload_kernels(void) {
   GL_NVTX("gl_preload_kernels");
   std::vector<const void *> funcs;
@@ -270,6 +271,9 @@ extern "C" int gl_preload_kernels(void) {
   gl_batch_kernels(funcs);
   gl_rader_kernels(funcs);
   gl_convolve_kernels(funcs);
+  gl_k12_kernels(funcs);
+  gl_permute_kernels(funcs);
+  gl_noalloc_kernels(funcs);
   for (const void *f : funcs) {
     cudaFuncAttributes attr;
     cudaError_t e = cudaFuncGetAttributes(&attr, f);

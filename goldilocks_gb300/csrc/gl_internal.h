@@ -85,11 +85,13 @@ void gl_launch_generic_fwd(const gl_pass_args &args, dim3 grid, cudaStream_t str
 void gl_launch_generic_inv(const gl_pass_args &args, dim3 grid, cudaStream_t stream, bool pdl);
 const void *gl_generic_kernel_fwd();
 const void *gl_generic_kernel_inv();
-// The other __global__ functions of the batch, Rader and convolution paths,
-// for gl_preload_kernels (gl_batch.cu, gl_rader.cu, gl_convolve.cu).
+// The other __global__ functions, for gl_preload_kernels (each in its own file).
 void gl_batch_kernels(std::vector<const void *> &out);
 void gl_rader_kernels(std::vector<const void *> &out);
 void gl_convolve_kernels(std::vector<const void *> &out);
+void gl_k12_kernels(std::vector<const void *> &out);
+void gl_permute_kernels(std::vector<const void *> &out);
+void gl_noalloc_kernels(std::vector<const void *> &out);
 #include "gl_generic.cuh"
 
 // Opt in to more than 48 KB of dynamic shared memory once per kernel and

@@ -346,3 +346,14 @@ extern "C" int gl_pow_solve(const uint8_t *challenge, uint64_t threshold, uint64
   *nonce = found;
   return GL_OK;
 }
+
+void gl_k12_kernels(std::vector<const void *> &out) {
+  out.push_back((const void *)gl_k12_layer_kernel<false>);
+  out.push_back((const void *)gl_k12_layer_kernel<true>);
+  out.push_back((const void *)gl_k12_few_kernel<false>);
+  out.push_back((const void *)gl_k12_few_kernel<true>);
+  out.push_back((const void *)gl_k12_top_kernel);
+  out.push_back((const void *)gl_k12_many_kernel);
+  out.push_back((const void *)gl_pow_hashes_kernel);
+  out.push_back((const void *)gl_pow_search_kernel);
+}

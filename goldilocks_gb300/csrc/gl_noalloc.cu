@@ -138,3 +138,5 @@ extern "C" int gl_ntt_noalloc(uint64_t *data, uint64_t len, int dir, void *strea
 
   return gl_cuda_status(cudaGetLastError());
 }
+
+void gl_noalloc_kernels(std::vector<const void *> &out) { out.push_back((const void *)fill_tables); }

@@ -100,3 +100,8 @@ extern "C" int gl_bit_reverse(uint64_t *data, uint64_t n, int mem, void *stream_
     return gl_cuda_status(cudaGetLastError());
   });
 }
+
+void gl_permute_kernels(std::vector<const void *> &out) {
+  out.push_back((const void *)transpose_kernel);
+  out.push_back((const void *)bit_reverse_kernel);
+}

@@ -349,8 +349,9 @@ int gl_transpose(uint64_t *data, uint64_t rows, uint64_t cols, int mem, void *st
  * (ntt/src/permute/mod.rs:70-74, permutation.rs:11-15). */
 int gl_bit_reverse(uint64_t *data, uint64_t n, int mem, void *stream);
 
-/* Load every kernel of the library onto the current device now (no
- * counterpart in the reference).  Under CUDA's lazy module loading a kernel
+/* Load every kernel of the library (but the autotuner's and
+ * gl_debug_field_op's own) onto the current device now (no counterpart in the
+ * reference).  Under CUDA's lazy module loading a kernel
  * is loaded at its first launch, and that load waits for the work already
  * running on the device; a multi-stream caller that must not stall calls
  * this during set-up.  gl_server_create calls it. */
