@@ -946,11 +946,9 @@ extern "C" int gl_profile_read(gl_profile_entry *out, int cap) {
 
 static const uint64_t kMaxGridYZ = 65535;
 
-// Debug builds (-DGL_DEVICE_CHECKS): every pass launch gets the extents of
-// its input and output (in words from its pointers) and the device's check
-// word; gl_debug_check_status reads and clears it.
+// The device's check word of a debug build (GL_DBG_EXTENTS).
 #ifdef GL_DEVICE_CHECKS
-static uint32_t *dbg_word() {
+uint32_t *gl_dbg_word() {
   static std::mutex mu;
   static std::map<int, uint32_t *> words;
   int dev = 0;
@@ -965,10 +963,6 @@ static uint32_t *dbg_word() {
   }
   return it->second;
 }
-#define GL_DBG_EXTENTS(args, in_words, out_words) \
-  do { (args).dbg_in_words = (in_words); (args).dbg_out_words = (out_words); (args).dbg_err = dbg_word(); } while (0)
-#else
-#define GL_DBG_EXTENTS(args, in_words, out_words) do {} while (0)
 #endif
 
 extern "C" int gl_debug_checks_enabled(void) { return GL_DBG_CHECKS; }
@@ -977,7 +971,7 @@ extern "C" int gl_debug_check_status(uint32_t *flags) {
   if (!flags) return GL_ERR_INVALID;
   *flags = 0;
 #ifdef GL_DEVICE_CHECKS
-  uint32_t *w = dbg_word();
+  uint32_t *w = gl_dbg_word();
   if (!w) return GL_ERR_CUDA;
   cudaError_t e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaMemcpy(flags, w, sizeof(uint32_t), cudaMemcpyDeviceToHost);

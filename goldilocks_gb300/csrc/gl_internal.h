@@ -257,6 +257,17 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
 
 const gl_kernel_entry *gl_contiguous_pass(const gl_plan *pl, int s, int d, uint64_t lanes, uint64_t items);
 
+// Debug builds (-DGL_DEVICE_CHECKS): a launch gets the extents of its input and
+// output (in words from its pointers) and the device's check word, which
+// gl_debug_check_status reads and clears.
+#ifdef GL_DEVICE_CHECKS
+uint32_t *gl_dbg_word();
+#define GL_DBG_EXTENTS(args, in_words, out_words) \
+  do { (args).dbg_in_words = (in_words); (args).dbg_out_words = (out_words); (args).dbg_err = gl_dbg_word(); } while (0)
+#else
+#define GL_DBG_EXTENTS(args, in_words, out_words) do {} while (0)
+#endif
+
 // Queue a batch on the persistent kernel without waiting; the kernel's error
 // word (0 = success) is copied to *err_out afterwards.  (gl_batch.cu)
 int gl_batch_enqueue_persistent(const gl_poly *polys, uint64_t count, cudaStream_t stream,

@@ -89,9 +89,10 @@ struct gl_pass_args {
   int64_t mul_ls, mul_bs, mul_bs2;
 };
 
-// Debug builds check every global and shared-memory index the pass kernels
-// use against its extent; a violation sets a bit of *dbg_err and the access
-// is skipped, so nothing traps.  Normal builds compile the checks away.
+// Debug builds check every global and shared-memory index that the pass kernels
+// and the one-kernel Rader step use against its extent; a violation sets a bit
+// of *dbg_err and the access is skipped, so nothing traps.  Normal builds
+// compile the checks away.
 #ifdef GL_DEVICE_CHECKS
 #define GL_DBG_CHECKS 1
 #else
@@ -99,8 +100,8 @@ struct gl_pass_args {
 #endif
 enum : uint32_t { GL_DBG_IN = 1u, GL_DBG_OUT = 2u, GL_DBG_SMEM = 4u };
 
-__device__ __forceinline__ bool gl_dbg_ok(const gl_pass_args &a, int64_t off, uint64_t lim,
-                                          uint32_t bit) {
+template <class Args>
+__device__ __forceinline__ bool gl_dbg_ok(const Args &a, int64_t off, uint64_t lim, uint32_t bit) {
   if (!GL_DBG_CHECKS || lim == 0 || (off >= 0 && (uint64_t)off < lim)) return true;
   if (a.dbg_err) atomicOr(a.dbg_err, bit);
   return false;
@@ -115,10 +116,12 @@ __device__ __forceinline__ void gl_st_out(const gl_pass_args &a, uint64_t *p, ui
   if (gl_dbg_ok(a, p - a.out, a.dbg_out_words, GL_DBG_OUT)) *p = v;
 }
 // Shared-memory word i of a tile of `lim` words.
-__device__ __forceinline__ uint64_t gl_sm_ld(const gl_pass_args &a, const uint64_t *sm, int i, int lim) {
+template <class Args>
+__device__ __forceinline__ uint64_t gl_sm_ld(const Args &a, const uint64_t *sm, int i, int lim) {
   return gl_dbg_ok(a, i, (uint64_t)lim, GL_DBG_SMEM) ? sm[i] : 0;
 }
-__device__ __forceinline__ void gl_sm_st(const gl_pass_args &a, uint64_t *sm, int i, int lim, uint64_t v) {
+template <class Args>
+__device__ __forceinline__ void gl_sm_st(const Args &a, uint64_t *sm, int i, int lim, uint64_t v) {
   if (gl_dbg_ok(a, i, (uint64_t)lim, GL_DBG_SMEM)) sm[i] = v;
 }
 

@@ -237,6 +237,7 @@ int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C
       a.gpow = t->rader_gpow; a.gneg = t->rader_gneg;
       a.tw_f = tq->blk[0][0]; a.tw_i = tq->blk_scaled_inv; a.bhat = t->rader_bhat[d];
       a.tw_lo = t->rader_tw_lo[d]; a.tw_hi = t->rader_tw_hi[d];
+      GL_DBG_EXTENTS(a, 257 * L, 257 * L);
       if ((st = rader257(a, stream, b > 0)) != GL_OK) return st;
       if (m > 1 && (st = gl_enqueue_transform(pl->pm, Y, out, q * C, 1, n * C, inv, sub, stream)) != GL_OK)
         return st;

@@ -25,6 +25,9 @@ struct gl_rader257_args {
   const uint64_t *tw_i;  // omega_256^-e / 256 (Montgomery form)
   const uint64_t *bhat;  // transformed Rader kernel (Montgomery form)
   const uint64_t *tw_lo, *tw_hi;  // omega_n^e (Montgomery form, perhaps scaled)
+  // Debug builds: the extents of src and dst in words (0: unchecked), the check word.
+  uint64_t dbg_in_words, dbg_out_words;
+  uint32_t *dbg_err;
 };
 
 template <int LN>
@@ -34,16 +37,22 @@ __device__ __forceinline__ void gl_rader257_block(const gl_rader257_args &a, uin
   const bool live = l < a.L;
   gl_pdl_launch_dependents();
   gl_pdl_wait();
+  constexpr int SM = LN * 272;
+  auto load = [&](const uint64_t *p) { return gl_dbg_ok(a, p - a.src, a.dbg_in_words, GL_DBG_IN) ? *p : 0; };
+  auto store = [&](uint64_t *p, uint64_t v) {
+    if (gl_dbg_ok(a, p - a.dst, a.dbg_out_words, GL_DBG_OUT)) *p = v;
+  };
   uint64_t x[16];
-  const uint64_t x0 = live ? gl_canon(a.src[l]) : 0;
+  const uint64_t x0 = live ? gl_canon(load(a.src + l)) : 0;
 #pragma unroll
-  for (int t = 0; t < 16; t++) x[t] = live ? a.src[__ldg(a.gpow + g + 16 * t) * a.L + l] : 0;
+  for (int t = 0; t < 16; t++) x[t] = live ? load(a.src + (__ldg(a.gpow + g + 16 * t) * a.L + l)) : 0;
   gl_dft_lazy<16, false>(x);
 #pragma unroll
-  for (int t = 0; t < 16; t++) sm[(t * 17 + g) * LN + c] = t ? gl_mont_mul(x[t], __ldg(a.tw_f + g * t)) : x[t];
+  for (int t = 0; t < 16; t++)
+    gl_sm_st(a, sm, (t * 17 + g) * LN + c, SM, t ? gl_mont_mul(x[t], __ldg(a.tw_f + g * t)) : x[t]);
   __syncthreads();
 #pragma unroll
-  for (int t = 0; t < 16; t++) x[t] = sm[(g * 17 + t) * LN + c];
+  for (int t = 0; t < 16; t++) x[t] = gl_sm_ld(a, sm, (g * 17 + t) * LN + c, SM);
   gl_dft_lazy<16, false>(x);
   // Frequency k = g + 16 t; that of k = 0 is the sum of all inputs but x[0].
   const uint64_t sum = gl_add(x0, gl_canon(x[0]));
@@ -52,10 +61,11 @@ __device__ __forceinline__ void gl_rader257_block(const gl_rader257_args &a, uin
   gl_dft_lazy<16, true>(x);
   __syncthreads();
 #pragma unroll
-  for (int t = 0; t < 16; t++) sm[(t * 17 + g) * LN + c] = gl_mont_mul(x[t], __ldg(a.tw_i + g * t));
+  for (int t = 0; t < 16; t++)
+    gl_sm_st(a, sm, (t * 17 + g) * LN + c, SM, gl_mont_mul(x[t], __ldg(a.tw_i + g * t)));
   __syncthreads();
 #pragma unroll
-  for (int t = 0; t < 16; t++) x[t] = sm[(g * 17 + t) * LN + c];
+  for (int t = 0; t < 16; t++) x[t] = gl_sm_ld(a, sm, (g * 17 + t) * LN + c, SM);
   gl_dft_lazy<16, true>(x);
   // Convolution outputs p = g + 16 t.
   const uint64_t j2 = a.C == 1 ? l : l / a.C;
@@ -68,17 +78,17 @@ __device__ __forceinline__ void gl_rader257_block(const gl_rader257_args &a, uin
   for (int t = 0; t < 16; t++) {
     const uint32_t k1 = __ldg(a.gneg + g + 16 * t);
     const uint64_t v = live ? gl_mont_mul(gl_add(x0, gl_canon(x[t])), gl_tw2m(a.tw_lo, a.tw_hi, j2 * k1)) : 0;
-    if (block) sm[c * 257 + k1] = v;
-    else if (live) out[k1 * a.C] = v;
+    if (block) gl_sm_st(a, sm, c * 257 + k1, SM, v);
+    else if (live) store(out + k1 * a.C, v);
   }
   if (g == 0) {
     const uint64_t v = live ? gl_mont_mul(sum, gl_tw2m(a.tw_lo, a.tw_hi, 0)) : 0;
-    if (block) sm[c * 257] = v;
-    else if (live) out[0] = v;
+    if (block) gl_sm_st(a, sm, c * 257, SM, v);
+    else if (live) store(out, v);
   }
   if (!block) return;
   __syncthreads();
   const uint64_t first = bx * (LN * 257), end = a.L * 257;
   for (int i = threadIdx.x; i < LN * 257; i += LN * 16)
-    if (first + i < end) a.dst[first + i] = sm[i];
+    if (first + i < end) store(a.dst + first + i, gl_sm_ld(a, sm, i, SM));
 }
