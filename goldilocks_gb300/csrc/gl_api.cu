@@ -890,7 +890,7 @@ static std::string kernel_label(const gl_kernel_entry *k, int role) {
 
 // Launch `k` with optional event bracketing.  role: 0 full, 1 col, 2 row.
 void gl_launch(const gl_kernel_entry *k, int role, const gl_pass_args &a0, dim3 grid,
-               uint64_t elements, cudaStream_t stream, bool pdl) {
+               uint64_t elements, cudaStream_t stream, bool pdl, bool chained) {
   gl_pass_args a = a0;
   if (k->generic) { a.gen_r[0] = k->r1; a.gen_r[1] = k->r2; a.gen_r[2] = k->r3; }
   bool on;
@@ -900,7 +900,15 @@ void gl_launch(const gl_kernel_entry *k, int role, const gl_pass_args &a0, dim3 
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (on && cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone)
     on = false;
-  if (!on) { k->launch(a, grid, stream, pdl); return; }
+  if (!on) {
+    // A pass that waits lets the next kernel in late (GL_PF_LATE), but not one of
+    // few CTAs: it cannot crowd, and the longer chain hides its latency better
+    // (64 points over 128 columns, 4 CTAs, 12.8 -> 11.0 us, LDE of 48 to 96 14.6 ->
+    // 10.4); nor where no pass follows programmatically.
+    if (pdl && chained && (uint64_t)grid.x * grid.y * grid.z > 8) a.flags |= GL_PF_LATE;
+    k->launch(a, grid, stream, pdl);
+    return;
+  }
   gl_prof_rec r{k, role, elements, nullptr, nullptr};
   cudaEventCreate(&r.a);
   cudaEventCreate(&r.b);
@@ -987,8 +995,10 @@ extern "C" int gl_debug_check_status(uint32_t *flags) {
 // is, before it reads or writes anything but its plan's tables, which were
 // complete before the plan was handed out.  Back to back calls then overlap
 // one's launch with the other's last wave.  Measured on GB300, calls back to
-// back (us): 1 024 points 6.2 -> 3.3, 2^13 10.2 -> 6.4, 2^16 10.3 -> 8.0, 2^20
-// 22.6 -> 18.8, 1 052 672 58.1 -> 45.5, 2^16 x 64 columns 47.2 -> 44.4,
+// back (us): 1 024 points 6.2 -> 3.4, 2^13 10.2 -> 6.5, 2^16 10.3 -> 7.4, 2^18
+// 11.7 -> 7.9, 2^20 22.7 -> 19.0, 1 052 672 58.1 -> 45.5 (before its Rader step
+// was one kernel), 2^16 x 64 columns 47.2 -> 44.6, 2^19 14.6 -> 15.1, 8 704 x 64
+// columns 16.6 -> 19.6 (20 of 865 shapes of up to 2^21 words lose over 2 %),
 // 16 711 680 313.9 -> 305.7.  A launch of many waves gains nothing and the LDE's
 // (107 tiles an SM) ran 0.6 % slower, so those start plainly.  So does a call
 // inside a stream capture, where it would add a programmatic edge to a graph of
@@ -1206,15 +1216,6 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
     }
     return gl_cuda_status(cudaGetLastError());
   }
-  // About one column tile per SM: launched beside a row pass that leaves SMs
-  // free, the tiles crowd on those.  us, early -> not: 393 216 points (192 tiles)
-  // 17.6 -> 15.1, 2^18 (128) 13.4 -> 12.1, 2^19 (256) 15.6 -> 15.2, 327 680 (160)
-  // 14.4 -> 15.0; outside, 2^17 (64) 9.0 -> 11.0, 655 360 (320) 18.0 -> 19.1, and
-  // tiles of 32 or 64 threads do not crowd: 2^15 (128 of 64 points) 7.0 -> 10.7.
-  auto uneven = [&](uint64_t tiles) {
-    const uint64_t sms = (uint64_t)gl_sm_count();
-    return C == 1 && pl->n1 >= 512 && 6 * tiles >= 5 * sms && tiles <= 2 * sms;
-  };
   // Four-step: n = n1*n2, j = n2*j1 + j2, k = k1 + n1*k2.
   const uint64_t n1 = pl->n1, n2 = pl->n2;
   const bool wide = C == 1 && lo->host;
@@ -1245,7 +1246,7 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
     const uint64_t lanes1 = n2 * C;
     if (gl_tiles(lanes1, kc) > 0x7fffffffull) return GL_ERR_INVALID;
     gl_launch(kc, 1, a, dim3((unsigned)gl_tiles(lanes1, kc), (unsigned)cb),
-              cb * n * C, stream, off > 0 || (pdl(gl_tiles(lanes1, kc) * cb) && !uneven(gl_tiles(lanes1, kc) * cb)));
+              cb * n * C, stream, off > 0 || pdl(gl_tiles(lanes1, kc) * cb));
     // ROW: n2-point transforms along j2 for every (k1, c); transposed store.
     gl_pass_args b = base_args();
     b.in_limit = 0xffffffffu;  // zero padding applies to the first pass only

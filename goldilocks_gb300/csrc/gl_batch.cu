@@ -501,7 +501,7 @@ int run_buckets(const gl_poly *polys, uint64_t count, const std::vector<poly_pla
         row.in_ptrs = (const uint64_t *const *)(dt + base_sc + j);
         row.out_ptrs = (uint64_t *const *)(dt + j);
         gl_launch(kr, 2, row, dim3((unsigned)gl_tiles(pl->n1, kr), (unsigned)(j1 - j)),
-                  pl->size * (j1 - j), on, true);
+                  pl->size * (j1 - j), on, true, false);
       }
       e = cudaGetLastError();
     }

@@ -9,18 +9,18 @@
 // Whether two polynomials of the batch share memory (length 1 is a no-op and
 // touches none).  A list in address order, as a packed pool's is, is one walk.
 inline bool gl_batch_shares_memory(const gl_poly *polys, uint64_t count) {
-  std::vector<std::pair<uint64_t, uint64_t>> spans;  // [first, end) in bytes
-  spans.reserve(count);
+  const auto first = [&](uint64_t i) { return (uint64_t)(uintptr_t)polys[i].data; };
   bool ordered = true;
-  uint64_t last = 0;
-  for (uint64_t i = 0; i < count; i++) {
+  uint64_t end = 0;
+  for (uint64_t i = 0; i < count && ordered; i++) {
     if (polys[i].len <= 1) continue;
-    const uint64_t first = (uint64_t)(uintptr_t)polys[i].data;
-    spans.push_back({first, first + 8 * polys[i].len});
-    ordered = ordered && first >= last;
-    last = spans.back().second;
+    ordered = first(i) >= end;
+    end = first(i) + 8 * polys[i].len;
   }
   if (ordered) return false;
+  std::vector<std::pair<uint64_t, uint64_t>> spans;  // [first, end) in bytes
+  for (uint64_t i = 0; i < count; i++)
+    if (polys[i].len > 1) spans.push_back({first(i), first(i) + 8 * polys[i].len});
   std::sort(spans.begin(), spans.end());
   for (size_t i = 1; i < spans.size(); i++)
     if (spans[i].first < spans[i - 1].second) return true;

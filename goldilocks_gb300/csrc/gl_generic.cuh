@@ -161,8 +161,9 @@ __device__ __forceinline__ void gl_gen_round_last(const gl_pass_args &a, const g
 template <bool INV>
 __global__ void __launch_bounds__(GL_GEN_NT) gl_generic_kernel(const gl_pass_args a) {
   extern __shared__ uint64_t sm[];
-  gl_pdl_launch_dependents();
+  if (!(a.flags & GL_PF_LATE)) gl_pdl_launch_dependents();
   gl_pdl_wait();
+  if (a.flags & GL_PF_LATE) gl_pdl_launch_dependents();
   gl_gen_ctx q;
   q.R1 = a.gen_r[0]; q.R2 = a.gen_r[1]; q.R3 = a.gen_r[2];
   q.M = q.R1 * q.R2 * q.R3;

@@ -187,9 +187,10 @@ int gl_table_upload(gl_dev_tables &t, const void *h, size_t bytes, void **dst);
 int gl_table_sync();
 void gl_table_free(std::vector<void *> &owned);
 // Launch `k` (optionally bracketed by profiling events).  role: 0 full,
-// 1 col, 2 row; pdl as for gl_launch_fn.
+// 1 col, 2 row; pdl as for gl_launch_fn; chained: the next kernel of the stream
+// may be launched with pdl, too.
 void gl_launch(const gl_kernel_entry *k, int role, const gl_pass_args &a, dim3 grid,
-               uint64_t elements, cudaStream_t stream, bool pdl = false);
+               uint64_t elements, cudaStream_t stream, bool pdl = false, bool chained = true);
 int gl_cuda_status(cudaError_t e);
 void gl_init_mempool_once();
 int gl_sm_count();  // multiprocessors of the current device

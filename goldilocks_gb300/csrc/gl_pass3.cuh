@@ -152,7 +152,7 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   // to ten instructions per element.
   const uint32_t lane0 = (uint32_t)bx * LANES;
   auto column = [&](uint32_t lane) { return a.tw_lane_div == 1 ? lane : lane / a.tw_lane_div; };
-  gl_pdl_launch_dependents();
+  if (!(a.flags & GL_PF_LATE)) gl_pdl_launch_dependents();
 
   // Stage the tables (read after the barrier that ends round 1).  They come
   // from constant tables, so they are loaded before the wait below and their
@@ -180,6 +180,7 @@ __device__ __forceinline__ void gl_block3(const gl_pass_args &a, int64_t bx, int
   // Everything below reads data an earlier kernel of the stream may write,
   // or writes global memory.
   gl_pdl_wait();
+  if (a.flags & GL_PF_LATE) gl_pdl_launch_dependents();
 
   const bool ptr_table = (a.flags & GL_PF_PTR_TABLE) != 0;
   const uint64_t *in = ptr_table ? a.in_ptrs[by] + bz * a.in_bs2 : a.in + by * a.in_bs + bz * a.in_bs2;
