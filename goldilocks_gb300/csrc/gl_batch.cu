@@ -587,6 +587,7 @@ extern "C" int gl_batch_execute(const gl_poly *polys, uint64_t count, int mode, 
     mode = it != g_tuned.end() ? it->second : GL_BATCH_BUCKETS;  // the faster one untuned
   }
   if (gl_batch_shares_memory(polys, count)) return run_in_order(polys, count, pp, stream);
+  if (mode == GL_BATCH_PER_CALL) return run_per_call(polys, count, stream);  // AUTO's choice
   if (mode == GL_BATCH_PERSISTENT) return run_persistent(polys, count, pp, stream);
   return run_buckets(polys, count, pp, stream);
 }
