@@ -127,6 +127,7 @@ GL_ERR_IO = 10
 GL_ERR_VERIFY = 11
 GL_FORWARD, GL_INVERSE = 0, 1
 GL_FOP_ADD, GL_FOP_SUB, GL_FOP_CANON, GL_FOP_MONT_MUL, GL_FOP_MUL, GL_FOP_SHL = 0, 1, 3, 4, 5, 100
+GL_FOP_LAZY = 1000
 GL_MEM_HOST, GL_MEM_DEVICE = 0, 1
 
 _lib = None

@@ -287,9 +287,16 @@ int gl_debug_inject_alloc_failures(int count);
  * 84, 96, 108, 144; b may be null).  The results are canonical.  Operand
  * contracts are those of gl_field.cuh: gl_add needs both operands below p,
  * gl_sub and gl_mont_mul the second, 2^96 (a negation) its operand; the
- * others take any words. */
+ * others take any words.
+ * GL_FOP_LAZY + 2*f + part: the codelets' operations on three 32-bit limbs, the
+ * top one signed; part 0 is the low word of the result, part 1 its top limb.
+ * With x = (a[i], top limb b[i] >> 32) and y = (b[i], top limb the low half of
+ * a[i]): f = 0 x + y, 1 x - y, 2 a + b, 3 a - b (words), 4 x + 12345 p, 5 12345 p
+ * - x, 6 x with its top limb folded in, 7 x >= 0 folded to a word, 8 + k x * 2^k
+ * (k in 3, 12, 24, 30, 32, 36, 48, 60, 63, 64, 72, 84, 93). */
 enum {
-  GL_FOP_ADD = 0, GL_FOP_SUB = 1, GL_FOP_CANON = 3, GL_FOP_MONT_MUL = 4, GL_FOP_MUL = 5, GL_FOP_SHL = 100
+  GL_FOP_ADD = 0, GL_FOP_SUB = 1, GL_FOP_CANON = 3, GL_FOP_MONT_MUL = 4, GL_FOP_MUL = 5, GL_FOP_SHL = 100,
+  GL_FOP_LAZY = 1000
 };
 int gl_debug_field_op(int op, const uint64_t *a, const uint64_t *b, uint64_t *out, uint64_t n, void *stream);
 
