@@ -55,8 +55,12 @@ def _buffer(values):
         if not values.is_contiguous():
             raise ValueError("device values must be contiguous")
         # The stream's handle without the torch.cuda.Stream object around it:
-        # the object was a third of a short call's host time.
-        stream = torch._C._cuda_getCurrentRawStream(values.get_device())
+        # the object was a third of a short call's host time.  The function is
+        # not public: a torch without it takes the object.
+        try:
+            stream = torch._C._cuda_getCurrentRawStream(values.get_device())
+        except AttributeError:
+            stream = torch.cuda.current_stream(values.device).cuda_stream
         return values.data_ptr(), values.numel(), L.GL_MEM_DEVICE, stream
     raise TypeError("values must be a numpy uint64 array or a CUDA torch tensor")
 
