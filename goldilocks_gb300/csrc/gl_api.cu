@@ -171,9 +171,9 @@ static const gl_kernel_entry *generic_entry(uint64_t m, bool inv) {
   e.threads = GL_GEN_NT;
   // Radices are still chosen at run time (and plans rank the size so), but
   // where a kernel is compiled for the size the launch goes to it.
-  const gl_kernel_entry *fixed = fixed_radix_entry(m, inv);
+  e.fixed = fixed_radix_entry(m, inv);
   static_assert(GL_GEN_LANES == 4, "the compiled kernels of these sizes have four lanes");
-  e.launch = fixed ? fixed->launch : inv ? gl_launch_generic_inv : gl_launch_generic_fwd;
+  e.launch = e.fixed ? e.fixed->launch : inv ? gl_launch_generic_inv : gl_launch_generic_fwd;
   e.generic = true;
   return &cache.emplace(key, e).first->second;
 }
@@ -281,6 +281,9 @@ extern "C" int gl_preload_kernels(void) {
   }
   return GL_OK;
 }
+
+// The kernel that an entry's launches run.
+static const gl_kernel_entry *launched(const gl_kernel_entry *k) { return k->fixed ? k->fixed : k; }
 
 static std::string kernel_shape(const gl_kernel_entry *k) {
   std::string s = std::to_string(k->m) + " (" + std::to_string(k->r1) + "x" + std::to_string(k->r2);
@@ -842,7 +845,8 @@ extern "C" uint64_t gl_plan_len(const gl_plan *plan) { return plan ? plan->size 
 extern "C" int gl_plan_describe(const gl_plan *plan, char *buf, size_t cap) {
   if (!plan || !buf) return GL_ERR_INVALID;
   std::string s = plan->tree + " | gpu: ";
-  auto kname = [](const gl_kernel_entry *k) {
+  auto kname = [](const gl_kernel_entry *entry) {
+    const gl_kernel_entry *k = launched(entry);
     std::string t = kernel_shape(k);
     t.insert(t.size() - 1, ", " + std::to_string(k->lanes) + " lanes" + (k->generic ? ", run-time radices" : "") +
                                (k->gt ? ", Good-Thomas" : ""));
@@ -885,7 +889,7 @@ static std::vector<gl_prof_rec> g_prof;
 
 static std::string kernel_label(const gl_kernel_entry *k, int role) {
   static const char *roles[] = {"full", "col", "row"};
-  return std::string(roles[role]) + " " + kernel_shape(k) + (role == 0 && k->lanes == 1 ? " single" : "");
+  return std::string(roles[role]) + " " + kernel_shape(launched(k)) + (role == 0 && k->lanes == 1 ? " single" : "");
 }
 
 // Launch `k` with optional event bracketing.  role: 0 full, 1 col, 2 row.

@@ -50,6 +50,7 @@ struct gl_kernel_entry {
   const void *func = nullptr;  // the __global__ function (gl_preload_kernels)
   bool gt = false;             // Good-Thomas inner transform: no pass twiddle allowed
   const void *func2 = nullptr;  // a second form the launcher picks by the arguments, if there is one
+  const gl_kernel_entry *fixed = nullptr;  // generic: the compiled kernel that `launch` runs instead
 };
 
 // Kernel sets compiled in separate translation units (parallel build).

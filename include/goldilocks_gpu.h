@@ -80,7 +80,10 @@ void gl_plan_release(gl_plan *plan);
 /* Ntt::len, mod.rs:26. */
 uint64_t gl_plan_len(const gl_plan *plan);
 /* The reference's plan tree for this size (e.g. "CT(4096,4096)[CT(64,64)[...]]")
- * followed by the GPU schedule ("| gpu: col 4096 (64x64) + row 4096 (64x64)").
+ * followed by the GPU schedule ("| gpu: col 4096 (16x16x16, 4 lanes) + row 4096
+ * (16x16x16, 4 lanes)"): the passes and the kernel of each, where a launch of
+ * many tiles, interleaved columns or host memory may take a kernel of the same
+ * radices with more lanes or another number of threads.
  * Returns GL_OK, or GL_ERR_INVALID if `cap` is too small (output truncated). */
 int gl_plan_describe(const gl_plan *plan, char *buf, size_t cap);
 /* Bytes of device scratch gl_plan_execute_ws needs for `count` transforms. */
