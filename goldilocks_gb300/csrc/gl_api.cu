@@ -860,9 +860,15 @@ extern "C" int gl_plan_describe(const gl_plan *plan, char *buf, size_t cap) {
          kname(plan->k[2][0]);
   else {
     char sub[1024];
-    s += "rader " + std::to_string(plan->q) + " [conv " + std::to_string(plan->q - 1);
-    if (gl_plan_describe(plan->pq, sub, sizeof sub) == GL_OK) s += ": " + std::string(strstr(sub, "gpu: ") + 5);
-    s += "] then " + std::to_string(plan->size / plan->q);
+    s += "rader " + std::to_string(plan->q);
+    if (gl_rader_one_kernel(plan)) {
+      s += " (one kernel)";
+    } else {
+      s += " [conv " + std::to_string(plan->q - 1);
+      if (gl_plan_describe(plan->pq, sub, sizeof sub) == GL_OK) s += ": " + std::string(strstr(sub, "gpu: ") + 5);
+      s += "]";
+    }
+    s += " then " + std::to_string(plan->size / plan->q);
     if (gl_plan_describe(plan->pm, sub, sizeof sub) == GL_OK) s += ": " + std::string(strstr(sub, "gpu: ") + 5);
   }
   size_t n = std::min(cap - 1, s.size());
@@ -878,8 +884,7 @@ extern "C" uint64_t gl_plan_workspace_bytes(const gl_plan *plan, uint64_t count)
 // ---------------------------------------------------------------- profiling
 
 struct gl_prof_rec {
-  const gl_kernel_entry *k;
-  int col;  // role: 0 full, 1 col, 2 row
+  std::string name;
   uint64_t elements;
   cudaEvent_t a, b;
 };
@@ -892,19 +897,32 @@ static std::string kernel_label(const gl_kernel_entry *k, int role) {
   return std::string(roles[role]) + " " + kernel_shape(launched(k)) + (role == 0 && k->lanes == 1 ? " single" : "");
 }
 
+bool gl_prof_begin(cudaStream_t stream, cudaEvent_t *start) {
+  if (!g_prof_on.load(std::memory_order_relaxed)) return false;
+  // Launches captured into a CUDA graph are not bracketed: the graph would
+  // keep event nodes for events the profile destroys when it is reset.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone) return false;
+  cudaEventCreate(start);
+  cudaEventRecord(*start, stream);
+  return true;
+}
+
+void gl_prof_end(cudaStream_t stream, cudaEvent_t start, const std::string &name, uint64_t elements) {
+  gl_prof_rec r{name, elements, start, nullptr};
+  cudaEventCreate(&r.b);
+  cudaEventRecord(r.b, stream);
+  std::lock_guard<std::mutex> lk(g_prof_mu);
+  g_prof.push_back(r);
+}
+
 // Launch `k` with optional event bracketing.  role: 0 full, 1 col, 2 row.
 void gl_launch(const gl_kernel_entry *k, int role, const gl_pass_args &a0, dim3 grid,
                uint64_t elements, cudaStream_t stream, bool pdl, bool chained) {
   gl_pass_args a = a0;
   if (k->generic) { a.gen_r[0] = k->r1; a.gen_r[1] = k->r2; a.gen_r[2] = k->r3; }
-  bool on;
-  on = g_prof_on.load(std::memory_order_relaxed);
-  // Launches captured into a CUDA graph are not bracketed: the graph would
-  // keep event nodes for events the profile destroys when it is reset.
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (on && cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone)
-    on = false;
-  if (!on) {
+  cudaEvent_t start;
+  if (!gl_prof_begin(stream, &start)) {
     // A pass that waits lets the next kernel in late (GL_PF_LATE), but not one of
     // few CTAs: it cannot crowd, and the longer chain hides its latency better
     // (64 points over 128 columns, 4 CTAs, 12.8 -> 11.0 us, LDE of 48 to 96 14.6 ->
@@ -913,14 +931,8 @@ void gl_launch(const gl_kernel_entry *k, int role, const gl_pass_args &a0, dim3 
     k->launch(a, grid, stream, pdl);
     return;
   }
-  gl_prof_rec r{k, role, elements, nullptr, nullptr};
-  cudaEventCreate(&r.a);
-  cudaEventCreate(&r.b);
-  cudaEventRecord(r.a, stream);
   k->launch(a, grid, stream, false);
-  cudaEventRecord(r.b, stream);
-  std::lock_guard<std::mutex> lk(g_prof_mu);
-  g_prof.push_back(r);
+  gl_prof_end(stream, start, kernel_label(k, role), elements);
 }
 
 extern "C" int gl_profile_enable(int on) {
@@ -939,9 +951,8 @@ extern "C" int gl_profile_read(gl_profile_entry *out, int cap) {
     if (e != cudaSuccess) return -gl_cuda_status(e);
     float ms = 0;
     cudaEventElapsedTime(&ms, r.a, r.b);
-    std::string name = kernel_label(r.k, (int)r.col);
-    gl_profile_entry &en = agg[name];
-    snprintf(en.name, sizeof(en.name), "%s", name.c_str());
+    gl_profile_entry &en = agg[r.name];
+    snprintf(en.name, sizeof(en.name), "%s", r.name.c_str());
     en.launches += 1;
     en.elements += r.elements;
     en.total_ms += ms;

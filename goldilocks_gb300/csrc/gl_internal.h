@@ -192,6 +192,10 @@ void gl_table_free(std::vector<void *> &owned);
 // may be launched with pdl, too.
 void gl_launch(const gl_kernel_entry *k, int role, const gl_pass_args &a, dim3 grid,
                uint64_t elements, cudaStream_t stream, bool pdl = false, bool chained = true);
+// The same bracketing around another kernel's launch: gl_prof_begin records the
+// first event and returns true while the profile is on (the launch is then plain).
+bool gl_prof_begin(cudaStream_t stream, cudaEvent_t *start);
+void gl_prof_end(cudaStream_t stream, cudaEvent_t start, const std::string &name, uint64_t elements);
 int gl_cuda_status(cudaError_t e);
 void gl_init_mempool_once();
 int gl_sm_count();  // multiprocessors of the current device
@@ -237,6 +241,7 @@ uint64_t gl_plan_scratch_words(const gl_plan *pl, uint64_t C, uint64_t B);
 // Kind-4 plans (gl_rader.cu): the tables, and the transform (no load or store
 // options; items one after another, so the scratch is that of one item).
 int gl_rader_tables(gl_plan *pl, gl_dev_tables &t);
+bool gl_rader_one_kernel(const gl_plan *pl);  // the step over 257 as gl_rader257_kernel
 int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C, uint64_t B,
                      uint64_t bs, bool inv, uint64_t *scratch, cudaStream_t stream);
 uint64_t gl_rader_scratch_words(const gl_plan *pl, uint64_t C);

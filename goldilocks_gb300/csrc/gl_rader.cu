@@ -48,7 +48,11 @@ int upload(gl_dev_tables &t, const std::vector<T> &h, T **dst) {
 // Launched with programmatic stream serialization: every kernel of a Rader step
 // waits for the one before it in the stream before it touches data.
 template <typename... P, typename... A>
-int launch(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t stream, bool pdl, A... args) {
+int launch(const char *name, uint64_t elements, void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t stream,
+           bool pdl, A... args) {
+  cudaEvent_t start;
+  const bool profile = gl_prof_begin(stream, &start);
+  if (profile) pdl = false;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
@@ -58,7 +62,9 @@ int launch(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t stream, bool 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return gl_cuda_status(cudaLaunchKernelEx(&cfg, kern, (P)args...));
+  const int st = gl_cuda_status(cudaLaunchKernelEx(&cfg, kern, (P)args...));
+  if (profile) gl_prof_end(stream, start, name, elements);
+  return st;
 }
 
 }  // namespace
@@ -158,9 +164,11 @@ static int rader257(const gl_rader257_args &a, cudaStream_t stream, bool early) 
   const int lanes = a.L <= 8ull * (unsigned)gl_sm_count() ? 8 : 16;
   const uint64_t tiles = (a.L + lanes - 1) / lanes;
   const bool pdl = early || gl_first_pass_pdl(stream, tiles);
-  return launch(lanes == 8 ? gl_rader257_kernel<8> : gl_rader257_kernel<16>, dim3((unsigned)tiles), lanes * 16, stream,
-                pdl, a);
+  return launch("rader 257", 257 * a.L, lanes == 8 ? gl_rader257_kernel<8> : gl_rader257_kernel<16>,
+                dim3((unsigned)tiles), lanes * 16, stream, pdl, a);
 }
+
+bool gl_rader_one_kernel(const gl_plan *pl) { return pl->q == 257 && pl->pq->kind == 1; }
 
 int gl_rader_tables(gl_plan *pl, gl_dev_tables &t) {
   const uint64_t q = pl->q, n = pl->size, r = q - 1;
@@ -226,7 +234,7 @@ int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C
   // The fused kernel takes the one-pass tables of 256 points (a tuned plan of
   // 256 in two passes has others) and up to 2^31 - 1 tiles.
   gl_dev_tables *tq = nullptr;
-  const bool fused = q == 257 && pl->pq->kind == 1 && L / 16 < 0x7fffffffull;
+  const bool fused = gl_rader_one_kernel(pl) && L / 16 < 0x7fffffffull;
   if (fused && (st = gl_plan_tables(pl->pq, &tq)) != GL_OK) return st;
   for (uint64_t b = 0; b < B; b++) {
     const uint64_t *in = src + b * bs;
@@ -243,21 +251,22 @@ int gl_rader_enqueue(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64_t C
         return st;
       continue;
     }
-    if ((st = launch(gl_rader_gather_kernel, grid_for(q * L), 256, stream, b > 0 || gl_first_pass_pdl(stream, 0), in,
-                     A, x0, t->rader_gpow, L, q)) != GL_OK)
+    if ((st = launch("rader gather", q * L, gl_rader_gather_kernel, grid_for(q * L), 256, stream,
+                     b > 0 || gl_first_pass_pdl(stream, 0), in, A, x0, t->rader_gpow, L, q)) != GL_OK)
       return st;
     if ((st = gl_enqueue_transform(pl->pq, A, A, L, 1, r * L, false, sub, stream)) != GL_OK) return st;
-    if ((st = launch(gl_rader_pointwise_kernel, grid_for(r * L), 256, stream, true, A, x0, X0, t->rader_bhat[d], L,
-                     r)) != GL_OK)
+    if ((st = launch("rader product", r * L, gl_rader_pointwise_kernel, grid_for(r * L), 256, stream, true, A, x0, X0,
+                     t->rader_bhat[d], L, r)) != GL_OK)
       return st;
     if ((st = gl_enqueue_transform(pl->pq, A, A, L, 1, r * L, true, sub, stream)) != GL_OK) return st;
     uint64_t *target = m > 1 ? Y : out;
     if (C < 8)
-      st = launch(gl_rader_scatter_tiled_kernel, dim3((unsigned)((L + 31) / 32), (unsigned)((q + 31) / 32)),
-                  dim3(32, 8), stream, true, A, x0, X0, target, t->rader_kpos, t->rader_tw_lo[d], t->rader_tw_hi[d], C, L, q);
+      st = launch("rader scatter", q * L, gl_rader_scatter_tiled_kernel,
+                  dim3((unsigned)((L + 31) / 32), (unsigned)((q + 31) / 32)), dim3(32, 8), stream, true, A, x0, X0,
+                  target, t->rader_kpos, t->rader_tw_lo[d], t->rader_tw_hi[d], C, L, q);
     else
-      st = launch(gl_rader_scatter_kernel, grid_for(q * L), 256, stream, true, A, x0, X0, target, t->rader_gneg,
-                  t->rader_tw_lo[d], t->rader_tw_hi[d], C, L, q);
+      st = launch("rader scatter", q * L, gl_rader_scatter_kernel, grid_for(q * L), 256, stream, true, A, x0, X0,
+                  target, t->rader_gneg, t->rader_tw_lo[d], t->rader_tw_hi[d], C, L, q);
     if (st != GL_OK) return st;
     if (m > 1 && (st = gl_enqueue_transform(pl->pm, Y, out, q * C, 1, n * C, inv, sub, stream)) != GL_OK)
       return st;

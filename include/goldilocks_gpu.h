@@ -438,8 +438,9 @@ typedef struct {
   double total_ms;     /* summed CUDA-event duration */
 } gl_profile_entry;
 
-/* While enabled, every kernel launch of the library is bracketed by CUDA
- * events on its own stream.  Enabling clears previous records. */
+/* While enabled, every launch of a transform's kernels (passes and Rader steps;
+ * not those inside a captured graph, the persistent batch kernel or a hash) is
+ * bracketed by CUDA events on its own stream.  Enabling clears previous records. */
 int gl_profile_enable(int on);
 /* Synchronises the recorded events and aggregates them by kernel; writes up
  * to `cap` entries and returns how many exist (or a negative gl_status). */

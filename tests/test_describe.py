@@ -26,6 +26,7 @@ def compiled():
     (15360, "col 128 (16x8x1, 4 lanes) + row 120 (15x8x1, 4 lanes)"),
     (61440, "col 256 (16x16x1, 4 lanes) + row 240 (16x15x1, 4 lanes)"),
     (1536, "full 1536 (16x16x6, 4 lanes)"),
+    (257 * 16, "rader 257 (one kernel) then 16: full 16 (16x1x1, 64 lanes)"),
     (48, "full 48 (16x3x1, 4 lanes, run-time radices)"),
 ])
 def test_pinned(gl, n, want):
