@@ -2,17 +2,19 @@
 // The same source compiles for the host (portable C++ branches) so that the
 // arithmetic and the generated codelets can be checked on a CPU; the device
 // branches are hand-written PTX carry chains on 32-bit halves, because the
-// integer ALU pipe (IADD3/SEL/SHF/ISETP) is the bottleneck of these kernels.
+// integer pipes bound these kernels (IADD3/SEL/SHF/ISETP on the ALU pipe, the
+// products' multiply-adds on the FMA pipe).
 //
-// Values are canonical u64 in [0, p).  The reference keeps the Montgomery form
-// x*2^64 mod p (ntt/src/field/mod.rs:12); every operation on the transform path
-// is F_p-linear, so the kernels work on either representation unchanged.
+// Values at rest are canonical u64 in [0, p).  The reference keeps the
+// Montgomery form x*2^64 mod p (ntt/src/field/mod.rs:12); every operation on the
+// transform path is F_p-linear, so the kernels work on either representation
+// unchanged.  Within a codelet values are three unreduced limbs ("lazy values").
 //
-// Multiplication is the 64x64->128 product (mul.lo / mul.hi) followed by the
-// reduction 2^64 = 2^32 - 1, 2^96 = -1 (mod p), restating reduce_159 of
-// ntt/src/field/algo/generic.rs:77-108.  Multiplications by powers of two --
-// the twiddles of order dividing 192 -- are shifts plus the same reduction
-// (generic.rs:171-193).
+// Multiplication is the 64x64->128 product followed by the reduction
+// 2^64 = 2^32 - 1, 2^96 = -1 (mod p), restating reduce_159 of
+// ntt/src/field/algo/generic.rs:77-108, or a Montgomery product by a table's
+// word.  Multiplications by powers of two -- the twiddles of order dividing 192
+// (generic.rs:171-193) -- shift the three limbs (gl_lshl).
 #pragma once
 #include <stdint.h>
 
@@ -126,39 +128,10 @@ GL_HD uint64_t gl_reduce159(uint64_t low, uint64_t mid, uint64_t high) {
 }
 
 #ifdef GL_DEV_PTX
-// A 32-bit constant the compiler cannot see through, so that multiplications
-// by it stay integer multiply-adds (FMA pipe) instead of becoming shifts (ALU).
-__device__ __forceinline__ uint32_t gl_opaque(uint32_t c) {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %1;" : "=r"(r) : "r"(c));
-  return r;
-}
-
 // value = (l1:l0) + h0*2^64 + h1*2^96 = (l1:l0) - h1 + h0*EPS (mod p), with
 // h0, h1 < 2^32; canonical result.
 __device__ __forceinline__ uint64_t gl_reduce_words(uint32_t l0, uint32_t l1, uint32_t h0,
                                                     uint32_t h1) {
-#ifdef GL_FIELD_V2
-  // h0*EPS as one 32x32->64 multiply (integer FMA pipe) instead of two ALU ops.
-  const uint64_t u = (uint64_t)h0 * gl_opaque(0xffffffffu);
-  uint32_t u0, u1;
-  gl_unpack(u, u0, u1);
-  uint32_t t0, t1, m, c;
-  asm("sub.cc.u32 %0, %4, %7;\n\t"       // t = l - h1
-      "subc.cc.u32 %1, %5, 0;\n\t"
-      "subc.u32 %2, 0, 0;\n\t"
-      "sub.cc.u32 %0, %0, %2;\n\t"       // borrow: + p
-      "subc.u32 %1, %1, 0;\n\t"
-      "add.cc.u32 %0, %0, %8;\n\t"       // t += u
-      "addc.cc.u32 %1, %1, %9;\n\t"
-      "addc.u32 %3, 0, 0;\n\t"
-      "sub.u32 %2, 0, %3;\n\t"           // carry: + EPS
-      "add.cc.u32 %0, %0, %2;\n\t"
-      "addc.u32 %1, %1, 0;"
-      : "=&r"(t0), "=&r"(t1), "=&r"(m), "=&r"(c)
-      : "r"(l0), "r"(l1), "r"(h0), "r"(h1), "r"(u0), "r"(u1));
-  return gl_canon32(t0, t1);
-#else
   uint32_t t0, t1, m, u0, u1, c;
   asm("sub.cc.u32 %0, %6, %9;\n\t"       // t = l - h1
       "subc.cc.u32 %1, %7, 0;\n\t"
@@ -176,7 +149,6 @@ __device__ __forceinline__ uint64_t gl_reduce_words(uint32_t l0, uint32_t l1, ui
       : "=&r"(t0), "=&r"(t1), "=&r"(m), "=&r"(u0), "=&r"(u1), "=&r"(c)
       : "r"(l0), "r"(l1), "r"(h0), "r"(h1));
   return gl_canon32(t0, t1);
-#endif
 }
 #endif
 
@@ -278,11 +250,9 @@ GL_HD constexpr uint64_t gl_pow2_mont(int k) {
   return x;
 }
 
-// x * 2^K mod p for a compile-time K in [0, 192).  By default a Montgomery
-// product by the constant 2^(K+64) mod p: about 11 operations on the integer
-// ALU pipe plus 8 multiply-adds on the FMA pipe, against about 21 ALU
-// operations for the word shifts and the canonical reduction below
-// (GL_SHL_WORDS) -- the ALU pipe is what bounds the transforms.
+// x * 2^K mod p for a compile-time K in [0, 192), canonical: on the device a
+// Montgomery product by the constant 2^(K+64) mod p.  (The codelets' shifts are
+// gl_lshl.)
 template <int K>
 GL_HD uint64_t gl_shl(uint64_t x) {
   static_assert(K >= 0 && K < 192, "shift out of range");
@@ -290,70 +260,14 @@ GL_HD uint64_t gl_shl(uint64_t x) {
     return x;
   } else if constexpr (K == 96) {
     return gl_neg(x);                     // 2^96 = -1
-#if defined(GL_DEV_PTX) && !defined(GL_SHL_WORDS)
-  } else if constexpr (true) {
-    constexpr uint64_t c = gl_pow2_mont(K);
-    return gl_mont_mul(x, c);
-#endif
-  } else if constexpr (K > 96) {
-    return gl_neg(gl_shl<K - 96>(x));     // 2^96 = -1
   } else {
 #ifdef GL_DEV_PTX
-    // x*2^K as words (w0..w3) of a 160-bit number, then
-    // value = (w1:w0) + w2*2^64 + w3*2^96 with w2, w3 < 2^32.
-    uint32_t x0, x1;
-    gl_unpack(x, x0, x1);
-    uint32_t w0, w1, w2, w3;
-#ifdef GL_FIELD_V2
-    if constexpr (K < 32 || (K > 32 && K < 64) || (K > 64 && K < 96)) {
-      // x * 2^s (s = K mod 32) as 32x32->64 multiply-adds on the FMA pipe.
-      constexpr int sh = K % 32;
-      const uint32_t c = gl_opaque(1u << sh);
-      const uint64_t p0 = (uint64_t)x0 * c;
-      const uint64_t p1 = (uint64_t)x1 * c + (p0 >> 32);
-      const uint32_t a0 = (uint32_t)p0, a1 = (uint32_t)p1, a2 = (uint32_t)(p1 >> 32);
-      if constexpr (K < 32) {
-        w0 = a0; w1 = a1; w2 = a2; w3 = 0;
-      } else if constexpr (K < 64) {
-        w0 = 0; w1 = a0; w2 = a1; w3 = a2;
-      } else {
-        // 64 < K < 96: x*2^K = a0*2^64 + a1*2^96 + a2*2^128, 2^128 = -2^32.
-        return gl_reduce_words(1u, 0xffffffffu - a2, a0, a1);
-      }
-      return gl_reduce_words(w0, w1, w2, w3);
-    }
-#endif
-    if constexpr (K < 32) {
-      w0 = x0 << K;
-      w1 = __funnelshift_l(x0, x1, K);
-      w2 = x1 >> (32 - K);
-      w3 = 0;
-    } else if constexpr (K == 32) {
-      w0 = 0; w1 = x0; w2 = x1; w3 = 0;
-    } else if constexpr (K < 64) {
-      w0 = 0;
-      w1 = x0 << (K - 32);
-      w2 = __funnelshift_l(x0, x1, K - 32);
-      w3 = x1 >> (64 - K);
-    } else if constexpr (K == 64) {
-      w0 = 0; w1 = 0; w2 = x0; w3 = x1;
-    } else {
-      w0 = 0;
-      w1 = 0;
-      w2 = x0 << (K - 64);
-      w3 = __funnelshift_l(x0, x1, K - 64);
-    }
-    if constexpr (K > 64) {
-      // 64 < K < 96: x*2^K = w2*2^64 + w3*2^96 + w4*2^128, w4 = x1 >> (96-K);
-      // 2^128 = 2^32 * 2^96 = -2^32, so w4*2^128 = -w4*2^32 (w4 < 2^31).
-      const uint32_t w4 = x1 >> (96 - K);
-      // -w4*2^32 + p as words (1, 0xffffffff - w4), then + w2*2^64 + w3*2^96.
-      return gl_reduce_words(1u, 0xffffffffu - w4, w2, w3);
-    } else {
-      return gl_reduce_words(w0, w1, w2, w3);
-    }
+    constexpr uint64_t c = gl_pow2_mont(K);
+    return gl_mont_mul(x, c);
 #else
-    if constexpr (K < 64) {
+    if constexpr (K > 96) {
+      return gl_neg(gl_shl<K - 96>(x));   // 2^96 = -1
+    } else if constexpr (K < 64) {
       uint64_t hi = x >> (64 - K);
       return gl_reduce159(x << K, hi & 0xffffffffull, hi >> 32);
     } else {

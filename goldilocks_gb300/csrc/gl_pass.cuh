@@ -163,7 +163,3 @@ __device__ __forceinline__ uint64_t gl_out_mul(const gl_pass_args &a, const uint
   v = gl_mul(v, __ldg(mb + lane * a.mul_ls + k * a.out_is));
   return (a.flags & GL_PF_OUT_MUL_MONT) ? gl_shl<128>(v) : v;  // 2^128 = 2^-64
 }
-
-__device__ __forceinline__ uint64_t gl_tw2(const uint64_t *lo, const uint64_t *hi, uint64_t e) {
-  return gl_mul(lo[e & 4095], hi[e >> 12]);
-}
