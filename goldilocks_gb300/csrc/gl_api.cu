@@ -968,6 +968,9 @@ extern "C" int gl_profile_read(gl_profile_entry *out, int cap) {
 // ---------------------------------------------------------------- execution
 
 static const uint64_t kMaxGridYZ = 65535;
+// Lanes of one launch of a single pass: a multiple of every kernel's lanes, and
+// 32-bit lane numbers do not wrap in the last tile.
+static const uint64_t kMaxLanes = 0xffffff00ull;
 
 // The device's check word of a debug build (GL_DBG_EXTENTS).
 #ifdef GL_DEVICE_CHECKS
@@ -1122,7 +1125,7 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
       a.in_ls = a.out_ls = (int64_t)bs; a.in_is = 1; a.out_is = (int64_t)Co;
       if (coset) { a.itw_jmul = 1; a.tw_lane_div = 0xffffffffu; }
       if (om) { a.flags |= mul_flags; a.mul_ls = mul_item; }  // lane = batch item
-      const uint64_t per = (uint64_t)k->lanes * 0x7fffffffull;
+      const uint64_t per = std::min<uint64_t>(k->lanes * 0x7fffffffull, kMaxLanes);
       const bool early = pdl(gl_tiles(B, k));
       for (uint64_t off = 0; off < B; off += per) {
         const uint64_t c = std::min(per, B - off);
@@ -1138,14 +1141,17 @@ int gl_enqueue_transform(gl_plan *pl, const uint64_t *src, uint64_t *dst, uint64
       a.in_bs = a.out_bs = (int64_t)bs;
       a.flags |= GL_PF_LOAD_LANE_FAST | GL_PF_STORE_LANE_FAST;
       if (coset) { a.itw_jmul = 1; a.tw_lane_div = 0xffffffffu; }
-      a.lanes = (uint32_t)C;
+      const uint64_t per = std::min<uint64_t>(k->lanes * 0x7fffffffull, kMaxLanes);
       const bool early = pdl(gl_tiles(C, k) * B);
       for (uint64_t off = 0; off < B; off += kMaxGridYZ) {
         const uint64_t c = std::min(kMaxGridYZ, B - off);
-        a.in = src + off * bs; a.out = dst + off * bs;
-        GL_DBG_EXTENTS(a, (c - 1) * bs + n * C, (c - 1) * bs + out_ext);
-        gl_launch(k, 0, a, dim3((unsigned)((C + k->lanes - 1) / k->lanes), (unsigned)c),
-               c * n * C, stream, early);
+        for (uint64_t col = 0; col < C; col += per) {
+          const uint64_t cols = std::min(per, C - col);
+          a.in = src + off * bs + col; a.out = dst + off * bs + col;
+          a.lanes = (uint32_t)cols;
+          GL_DBG_EXTENTS(a, (c - 1) * bs + n * C - col, (c - 1) * bs + out_ext - col);
+          gl_launch(k, 0, a, dim3((unsigned)gl_tiles(cols, k), (unsigned)c), c * n * cols, stream, early);
+        }
       }
     }
     return gl_cuda_status(cudaGetLastError());
