@@ -158,8 +158,11 @@ __global__ void __launch_bounds__(LN * 16, 64 / LN) gl_rader257_kernel(const gl_
 }
 
 // Eight lanes while they give every SM at most one tile, else sixteen (128-byte
-// rows).  us, 16 -> 8 lanes: 257 x 1024 23.8 -> 21.8, 257 12.6 -> 11.4, 257 x 64 26.9 ->
-// 28.2; 257 x 3840 48.9 -> 50.0, 257 x 65536 361 -> 374 (four lanes 378).
+// rows).  Whole transforms of 257 x m points or over columns, 68 shapes of up to
+// 1 216 lanes, 16 lanes -> 8 (us): 2 % faster in the mean, one 257 12.0 -> 10.4,
+// over 1 000 columns 12.2 -> 11.4, 257 x 1024 even; 257 x 15 (25.3 -> 26.3) and 257 x
+// 20 (17.5 -> 19.6) lose most.  Above: 257 x 1536 24.5 -> 22.6, 257 x 3840 48.9 ->
+// 50.0, 257 x 65536 361 -> 374 (four lanes 378).
 static int rader257(const gl_rader257_args &a, cudaStream_t stream, bool early) {
   const int lanes = a.L <= 8ull * (unsigned)gl_sm_count() ? 8 : 16;
   const uint64_t tiles = (a.L + lanes - 1) / lanes;
