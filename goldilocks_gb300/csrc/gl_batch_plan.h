@@ -7,21 +7,36 @@
 #include "../../include/goldilocks_gpu.h"
 
 // Whether two polynomials of the batch share memory (length 1 is a no-op and
-// touches none).  A list in address order, as a packed pool's is, is one walk.
+// touches none).  A list in address order, as a packed pool's is, is one walk;
+// any other is sorted into about two cells of the address range per polynomial
+// first (1 024 in random order: std::sort alone took 28 us of a 920 us batch).
 inline bool gl_batch_shares_memory(const gl_poly *polys, uint64_t count) {
   const auto first = [&](uint64_t i) { return (uint64_t)(uintptr_t)polys[i].data; };
   bool ordered = true;
-  uint64_t end = 0;
-  for (uint64_t i = 0; i < count && ordered; i++) {
+  uint64_t lo = ~0ull, hi = 0, last = 0, total = 0, n = 0;
+  for (uint64_t i = 0; i < count; i++) {
     if (polys[i].len <= 1) continue;
-    ordered = first(i) >= end;
-    end = first(i) + 8 * polys[i].len;
+    const uint64_t end = first(i) + 8 * polys[i].len;
+    ordered = ordered && first(i) >= last;
+    last = end;
+    lo = std::min(lo, first(i));
+    hi = std::max(hi, end);
+    total += 8 * polys[i].len;
+    n++;
   }
   if (ordered) return false;
-  std::vector<std::pair<uint64_t, uint64_t>> spans;  // [first, end) in bytes
+  if (total > hi - lo) return true;
+  int shift = 0;
+  while ((hi - lo) >> shift >= 2 * n) shift++;
+  std::vector<uint32_t> at(((hi - lo) >> shift) + 2, 0);  // where each cell starts
   for (uint64_t i = 0; i < count; i++)
-    if (polys[i].len > 1) spans.push_back({first(i), first(i) + 8 * polys[i].len});
-  std::sort(spans.begin(), spans.end());
+    if (polys[i].len > 1) at[((first(i) - lo) >> shift) + 1]++;
+  for (size_t c = 1; c < at.size(); c++) at[c] += at[c - 1];
+  std::vector<std::pair<uint64_t, uint64_t>> spans(n);  // [first, end) in bytes
+  for (uint64_t i = 0; i < count; i++)
+    if (polys[i].len > 1) spans[at[(first(i) - lo) >> shift]++] = {first(i), first(i) + 8 * polys[i].len};
+  for (size_t c = 0, a = 0; c + 1 < at.size(); a = at[c++])  // at[c] is now where cell c ends
+    if (at[c] > a + 1) std::sort(spans.begin() + a, spans.begin() + at[c]);
   for (size_t i = 1; i < spans.size(); i++)
     if (spans[i].first < spans[i - 1].second) return true;
   return false;

@@ -54,6 +54,21 @@ def test_sharing_is_found(plan):
     assert seen == {True, False}
 
 
+def test_sharing_is_found_in_any_order_and_spread(plan):
+    rng = random.Random(2)
+    seen = {True: 0, False: 0}
+    for _ in range(600):
+        reach = 1 << rng.randrange(6, 40)
+        spans = [(rng.randrange(reach), rng.randrange(1, 2 + reach // rng.randrange(8, 4000)), 0)
+                 for _ in range(rng.randrange(2, 60))]
+        ends = sorted((at, at + n) for at, n, _ in spans if n > 1)
+        want = any(b[0] < a[1] for a, b in zip(ends, ends[1:]))
+        arr = polys(spans)
+        assert bool(plan.shares(ctypes.byref(arr), ctypes.c_uint64(len(spans)))) == want, spans
+        seen[want] += 1
+    assert min(seen.values()) > 50
+
+
 def test_order(plan):
     spans = [(0, 16, 1), (0, 8, 0), (0, 64, 0), (0, 16, 0), (0, 8, 1), (0, 32, 1), (0, 8, 0), (0, 16, 0)]
     plain = np.array([0, 0, 1, 0, 0, 1, 0, 0], dtype=np.uint8)
